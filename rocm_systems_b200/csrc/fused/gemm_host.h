@@ -14,4 +14,13 @@ int smCount();
 cudaError_t gemmBf16TN(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int bn, int maxCtas, cudaStream_t s);
 
 }  // namespace gemm
+namespace gemm2 {
+int pairsOnDevice();
+cudaError_t gemmPairBf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, bool aMn, bool bMn, int bn, int maxCtas,
+                         cudaStream_t s);
+}  // namespace gemm2
+namespace gemmn {
+bool prefersNarrow(int M, int N);
+cudaError_t gemmNarrowBf16(const void* X, const void* W, void* C, int M, int N, int K, int ldx, int ldw, int ldc, bool wMn, int gateUpTile, cudaStream_t s);
+}  // namespace gemmn
 }  // namespace b200

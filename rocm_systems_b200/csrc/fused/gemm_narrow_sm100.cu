@@ -1,0 +1,87 @@
+// Host side of the few-row bf16 GEMM (gemm_narrow_sm100.cuh): which shapes it takes, tile and split choice, cluster launch.
+#include "gemm_narrow_sm100.cuh"
+
+#include <algorithm>
+
+#include "gemm_host.h"
+
+namespace b200 {
+namespace gemmn {
+namespace {
+
+template <int TN, bool W_MN, bool SWIGLU>
+cudaError_t launch(const Params& p, int tiles, int S, cudaStream_t s) {
+  auto kernel = gemmNarrowKernel<TN, W_MN, SWIGLU>;
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<TN>::kSmemBytes);
+    if (e != cudaSuccess) return e;
+    configured[dev] = true;
+  }
+  cudaLaunchConfig_t q{};
+  q.gridDim = dim3((unsigned)(S * tiles), (unsigned)((p.M + TN - 1) / TN));
+  q.blockDim = dim3(kThreads);
+  q.dynamicSmemBytes = Cfg<TN>::kSmemBytes;
+  q.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)S;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = 1;
+  q.attrs = &at;
+  q.numAttrs = S > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&q, kernel, p, S);
+}
+
+template <bool W_MN, bool SWIGLU>
+cudaError_t dispatch(const Params& p, int tn, int tiles, int S, cudaStream_t s) {
+  switch (tn) {
+    case 16: return launch<16, W_MN, SWIGLU>(p, tiles, S, s);
+    case 32: return launch<32, W_MN, SWIGLU>(p, tiles, S, s);
+    case 64: return launch<64, W_MN, SWIGLU>(p, tiles, S, s);
+    default: return launch<128, W_MN, SWIGLU>(p, tiles, S, s);
+  }
+}
+
+}  // namespace
+
+// Where this kernel is the faster one, measured over M 1 .. 1024, N 1024 .. 28672, K 512 .. 14336 with the weights out of
+// the L2. Up to 128 rows everywhere (N 28672, K 4096, 128 rows: 48 us against 56 on CTA pairs; N 1024, K 512: 4 - 5 against
+// 9). Above, W is read again for every 128 rows, and it pays only while the 256 x 256 tiles would leave half of the device
+// idle: 512 x 4096 x 4096 23 us against 27, 512 x 4096 x 14336 58 against 73, but 512 x 6144 x 4096 31 against 28. Above 512
+// rows never (768 x 4096 x 4096 30 against 28).
+bool prefersNarrow(int M, int N) {
+  if (M <= 128) return true;
+  const int tiles = ((M + 255) / 256) * ((N + 255) / 256);
+  return M <= 512 && 2 * tiles <= gemm2::pairsOnDevice();
+}
+
+// C [M, N or N / 2] = X [M, K] * W [N, K]^T; wMn: W is stored [K, N]. gateUpTile != 0: SwiGLU over the interleaved rows of W.
+cudaError_t gemmNarrowBf16(const void* X, const void* W, void* C, int M, int N, int K, int ldx, int ldw, int ldc, bool wMn, int gateUpTile, cudaStream_t s) {
+  Params p{};
+  const int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+  const bool okW = wMn ? gemm::makeTileMap(&p.mapW, W, K, N, ldw, 64, 2) : gemm::makeTileMap(&p.mapW, W, N, K, ldw, 64, 2);
+  if (!okW || !gemm::makeTileMap(&p.mapX, X, M, K, ldx, tn, 2)) return cudaErrorInvalidValue;
+  p.C = (__nv_bfloat16*)C;
+  p.ldc = ldc;
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.gateUpTile = gateUpTile;
+  p.err = gemm::errWord();
+  if (!p.err) return cudaErrorMemoryAllocation;
+  // Split K until the CTAs fill the device (two to an SM): 4096 x 4096 on 16 rows takes 14.8 us with 2 splits, 10.8 - 11.4 with
+  // 4 - 8. One token tile: at most 240 CTAs, because from 128 feature tiles up the exchange costs more than the second CTA of an
+  // SM gives (16384 x 2048 on 16 rows: 15.2 us unsplit, 16.1 in two). A cluster beyond that number waits for a second wave
+  // (6144 x 4096: 13.5 us with 240 CTAs, 18.6 with 288).
+  const int tiles = (N + BF - 1) / BF, tokTiles = (M + tn - 1) / tn, kIters = (K + BK - 1) / BK;
+  const int S = std::max(1, std::min({kMaxSplit, kIters, (tokTiles == 1 ? 240 : 256) / (tiles * tokTiles)}));
+  if (gateUpTile) return wMn ? cudaErrorInvalidValue : dispatch<false, true>(p, tn, tiles, S, s);
+  return wMn ? dispatch<true, false>(p, tn, tiles, S, s) : dispatch<false, false>(p, tn, tiles, S, s);
+}
+
+}  // namespace gemmn
+}  // namespace b200

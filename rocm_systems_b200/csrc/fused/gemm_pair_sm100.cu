@@ -71,6 +71,7 @@ cudaError_t gemmPairBf16(const void* A, const void* B, void* C, int M, int N, in
                          cudaStream_t s) {
   if (M <= 0 || N <= 0 || K <= 0) return cudaSuccess;
   if ((reinterpret_cast<uintptr_t>(C) & 15) || (ldc & 7)) return cudaErrorInvalidValue;  // rows of C are written in 16-byte pieces
+  if (bn == 0 && maxCtas == 0 && !aMn && gemmn::prefersNarrow(M, N)) return gemmn::gemmNarrowBf16(A, B, C, M, N, K, lda, ldb, ldc, bMn, 0, s);
   // 256-wide tiles unless the caller says otherwise: on 128-wide ones the issuing thread's per-stage work (barrier wait,
   // descriptors, commit) is no longer hidden behind the MMAs, and the kernel ran 1.6x slower on the same problem.
   if (bn != 128 && bn != 256) bn = N > 128 ? 256 : 128;
@@ -98,7 +99,7 @@ extern "C" {
 // CTA pairs the current device runs at once (what the tile-width choice divides the tiles by).
 int b200ops_gemm_pairs_on_device(void) { return b200::gemm2::pairsOnDevice(); }
 
-// C[M, N] (bf16, ldc) = A * B^T on CTA pairs. A is logical [M, K], B logical [N, K]; aMn / bMn != 0 says the operand is
+// C[M, N] (bf16, ldc) = A * B^T on CTA pairs, or for few rows on the kernel of gemm_narrow_sm100.cuh (bn and maxCtas 0). A is logical [M, K], B logical [N, K]; aMn / bMn != 0 says the operand is
 // stored with its row index contiguous ([K, M] resp. [K, N] row-major, leading dimension = the row stride of that
 // storage). bn: 0 auto, 128 or 256. Errors of bounded waits are read with b200ops_gemm_take_error.
 int b200ops_gemm_bf16_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int aMn, int bMn, int bn, int maxCtas,

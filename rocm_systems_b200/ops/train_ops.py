@@ -228,7 +228,8 @@ def gemm_bf16_tn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, bn:
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, bn: int = 0, max_ctas: int = 0) -> torch.Tensor:
-    """``a @ b.T`` in bf16 with fp32 accumulation on the CTA-pair tcgen05 kernel (csrc/fused/gemm_pair_sm100.cuh).
+    """``a @ b.T`` in bf16 with fp32 accumulation on the CTA-pair tcgen05 kernel (csrc/fused/gemm_pair_sm100.cuh), or for few
+    rows of a row-major ``a`` on the one that splits the reduction instead (csrc/fused/gemm_narrow_sm100.cuh).
 
     ``a`` is [M, K] and ``b`` [N, K] as tensors; each may be a row-major matrix or the transposed view of one
     (``x.t()``): the kernel reads either memory order directly (K-major or MN-major operand), so the three GEMMs of a

@@ -55,3 +55,26 @@ def test_gemm_on_cta_pairs_writes_into_a_strided_view():
     ref = a.float() @ b.float().t()
     assert (big[:, 64:264].float() - ref).abs().max().item() <= 1e-2 * ref.abs().max().item() + 1e-2
     assert bool((big[:, :64] == 7).all()) and bool((big[:, 264:] == 7).all())     # nothing outside the view was written
+
+
+@pytest.mark.parametrize("wt", [False, True])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (1, 1000, 8), (16, 6144, 4096), (17, 136, 200), (33, 4096, 14336), (64, 28672, 512), (65, 1032, 1000),
+                                   (128, 264, 328), (129, 4096, 1024), (300, 520, 4096), (512, 1024, 520)])
+def test_gemm_of_few_rows_matches_fp32(M, N, K, wt):
+    """Sizes that take the kernel with output features as MMA rows and K split over a cluster (one token up to four token tiles, ragged
+    edges in every direction, fewer 64-step slices than splits). Bound: one bf16 rounding of the result (2^-9 of its size) plus the
+    fp32 sums of both sides, K products of unit variance whose partial sums stay below 6 sqrt(K): 2 K 2^-24 6 sqrt(K) at the very worst,
+    a hundredth of it in practice."""
+    from rocm_systems_b200.ops import train_ops as ops
+
+    torch.manual_seed(M + N + K)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    w = torch.randn(K, N, device="cuda").to(torch.bfloat16).t() if wt else torch.randn(N, K, device="cuda").to(torch.bfloat16)
+    big = torch.full((M + 1, N + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.gemm(x, w, out=big[:M, :N])
+    torch.cuda.synchronize()
+    assert ops.gemm_take_error() == 0
+    ref = x.double() @ w.double().t()
+    err = (big[:M, :N].double() - ref).abs()
+    assert bool((err <= ref.abs() * 2.0 ** -8 + 1e-6 * K ** 0.5).all()), float((err - ref.abs() * 2.0 ** -8).max())
+    assert bool((big[M:] == 7).all()) and bool((big[:, N:] == 7).all())     # nothing outside the view was written
