@@ -321,6 +321,16 @@ ncclResult_t b200collAgGemm(ncclComm_t comm, void* xSym, const void* w, void* ou
   const int M = rowsPerRank * n;
   if (c->asyncError.load() != ncclSuccess) BFAIL((ncclResult_t)c->asyncError.load(), "communicator is in an error state: %s", c->lastErr.c_str());
   DevGuard2 g(c->cudaDev);
+  // One rank gathers nothing: the plain GEMMs take the call where they have its epilogue. Without SwiGLU that is the CTA-pair
+  // kernel (4096 x 4096 x 6144: 0.14 ms against 0.16 for the one-CTA kernel below); with it the few-row kernel, whose rule
+  // says where (128 x 28672 x 4096: 47 us against 49.5, and half the device stays idle on smaller weights).
+  if (n == 1 && (!swiglu || gemmn::prefersNarrow(M, wRows))) {
+    const cudaError_t e = swiglu ? gemmn::gemmNarrowBf16(xSym, w, out, M, wRows, K, K, K, wRows / 2, false, bn, stream)
+                                 : gemm2::gemmPairBf16(xSym, w, out, M, wRows, K, K, K, wRows, false, false, 0, 0, stream);
+    if (e == cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "b200collAgGemm: operands must be 16-byte aligned with rows a multiple of 16 bytes");
+    if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "b200collAgGemm launch failed: %s", cudaGetErrorString(e));
+    return ncclSuccess;
+  }
   AgArgs a{};
   char* peers[kMaxRanks] = {};
   if (n > 1) {
@@ -403,6 +413,14 @@ ncclResult_t b200collGemmRs(ncclComm_t comm, const void* a_, const void* w, void
   const size_t flags = (wsBytes - 2 * stage) / 2;
   unsigned long long calls;
   BCHECK(rsNextCall(c, workspaceSym, bn, &calls));
+  // One rank owns every row and has nobody's partial sums to add: the GEMM writes the result itself (staging and reducing a
+  // single partial took 0.15 ms of 0.55 on 4096 x 4096 x 14336, and the few-row kernel splits K where 128 rows would use 16 CTAs).
+  if (n == 1) {
+    const cudaError_t e = gemm2::gemmPairBf16(a_, w, y, M, N, K, K, K, N, false, false, 0, 0, stream);
+    if (e == cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "b200collGemmRs: operands must be 16-byte aligned with rows a multiple of 16 bytes");
+    if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "b200collGemmRs launch failed: %s", cudaGetErrorString(e));
+    return ncclSuccess;
+  }
   const int parity = (int)(calls & 1);
   a.stageOff = (size_t)parity * stage;
   a.flagOff = 2 * stage + (size_t)parity * flags;

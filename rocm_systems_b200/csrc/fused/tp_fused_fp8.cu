@@ -183,6 +183,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemmRsFp8Kernel(const __grid_cons
 using namespace b200;
 using namespace b200::tp8;
 
+extern "C" int b200ops_gemm_fp8_block_tn(const void* A8, const float* sA, const void* B8, const float* sB, void* C, int M, int N, int K, int lda, int ldb, int ldc,
+                                         int maxCtas, cudaStream_t st);
+
 extern "C" {
 
 ncclResult_t b200collAgGemmFp8(ncclComm_t comm, void* x8Sym, float* sASym, const void* w8, const float* sW, void* out, int rowsPerRank, int wRows, int K,
@@ -284,6 +287,12 @@ ncclResult_t b200collGemmRsFp8(ncclComm_t comm, const void* a8, const float* sA,
   const size_t flags = (wsBytes - 2 * stage) / 2;
   unsigned long long calls;
   BCHECK(tp::rsNextCall(c, workspaceSym, BN, &calls));
+  if (n == 1) {  // nobody's partial sums to add: the GEMM writes the result itself
+    const int e = b200ops_gemm_fp8_block_tn(a8, sA, w8, sW, y, M, N, K, K, K, N, 0, stream);
+    if (e == (int)cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "b200collGemmRsFp8: operands must be 16-byte aligned");
+    if (e) BFAIL(ncclUnhandledCudaError, "b200collGemmRsFp8 launch failed: %s", cudaGetErrorString((cudaError_t)e));
+    return ncclSuccess;
+  }
   const int parity = (int)(calls & 1);
   a.stageOff = (size_t)parity * stage;
   a.flagOff = 2 * stage + (size_t)parity * flags;
