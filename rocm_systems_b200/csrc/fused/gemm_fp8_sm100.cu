@@ -12,42 +12,38 @@ __global__ void __launch_bounds__(kThreads, 1) gemmFp8BlockKernel(const __grid_c
 }
 
 // ---- quantisers ------------------------------------------------------------------------------------------------
-// Activations: one scale per row and 128 channels. A warp takes a row; lane l holds channels (32 j + l) * 8 .. + 8 of
-// round j, so a half-warp is one 128-channel group.
-__global__ void __launch_bounds__(256) quantRows1x128(const __nv_bfloat16* x, uint8_t* q, float* s, int M, int K, int ldx, int ldq, int lds) {
+// Activations: one scale per row and 128 channels. A CTA takes 8 rows (a warp each, so that the 8 scales of a group, neighbours in
+// the table, go to one 32-byte sector) and up to 4 rounds of 256 channels: lane l holds channels (32 j + l) * 8 .. + 8 of round j, a
+// half-warp is one group, and all its loads are in flight at once. With a whole row per warp, one round after the other,
+// 32 rows of 14336 channels took 31 us, 56 round trips to memory; 4096 x 4096 took 20 us, half of it in the divisions.
+constexpr int kQuantRounds = 4;
+__global__ void __launch_bounds__(256) quantRows1x128(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ s, int M, int K, int ldx,
+                                                      int ldq, int lds) {
   const int lane = threadIdx.x & 31;
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  sm100::gridLaunchDependents();
   if (row >= M) return;
   const int groups = K / 128;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * ldx);
   uint2* qr = reinterpret_cast<uint2*>(q + (size_t)row * ldq);
-  for (int j = 0; j * 2 < groups; j++) {
-    const int g = j * 2 + (lane >> 4);
-    const bool live = g < groups;
-    uint4 raw = make_uint4(0, 0, 0, 0);
-    if (live) raw = xr[j * 32 + lane];
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-    float f[8];
-    float amax = 0.f;
+  const int j0 = blockIdx.y * kQuantRounds;
+  uint4 raw[kQuantRounds];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const float2 pr = __bfloat1622float2(h[i]);
-      f[2 * i] = pr.x;
-      f[2 * i + 1] = pr.y;
-      amax = fmaxf(amax, fmaxf(fabsf(pr.x), fabsf(pr.y)));
-    }
+  for (int j = 0; j < kQuantRounds; j++) {
+    raw[j] = make_uint4(0, 0, 0, 0);
+    if ((j0 + j) * 2 + (lane >> 4) < groups) raw[j] = xr[(j0 + j) * 32 + lane];
+  }
+#pragma unroll
+  for (int j = 0; j < kQuantRounds; j++) {
+    const int g = (j0 + j) * 2 + (lane >> 4);
+    float f[8], amax = 0.f;
+    unpackBf16x8(raw[j], f, amax);
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float scale = fmaxf(amax, 1e-10f) * (1.f / 448.f);
-    uint32_t w[2];
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const __nv_fp8x4_e4m3 p4(make_float4(__fdiv_rn(f[4 * i], scale), __fdiv_rn(f[4 * i + 1], scale), __fdiv_rn(f[4 * i + 2], scale), __fdiv_rn(f[4 * i + 3], scale)));
-      w[i] = *reinterpret_cast<const uint32_t*>(&p4);
-    }
-    if (live) {
-      qr[j * 32 + lane] = make_uint2(w[0], w[1]);
-      if ((lane & 15) == 0) s[(size_t)g * lds + row] = scale;
+    const QuantScale qs(amax);
+    if (g < groups) {
+      qr[(j0 + j) * 32 + lane] = qs.codes(f);
+      if ((lane & 15) == 0) s[(size_t)g * lds + row] = qs.scale;
     }
   }
 }
@@ -79,27 +75,15 @@ __global__ void __launch_bounds__(256) quantBlocks128x128(const __nv_bfloat16* w
   amax = red[0];
 #pragma unroll
   for (int i = 1; i < 8; i++) amax = fmaxf(amax, red[i]);
-  const float scale = fmaxf(amax, 1e-10f) * (1.f / 448.f);
-  if (t == 0) s[(size_t)nb * gridDim.x + kb] = scale;
+  const QuantScale qs(amax);
+  if (t == 0) s[(size_t)nb * gridDim.x + kb] = qs.scale;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     const int row = nb * 128 + r0 + 16 * i;
     if (row >= N) continue;
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[i]);
-    float f[8];
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const float2 pr = __bfloat1622float2(h[e]);
-      f[2 * e] = pr.x;
-      f[2 * e + 1] = pr.y;
-    }
-    uint32_t o[2];
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const __nv_fp8x4_e4m3 p4(make_float4(__fdiv_rn(f[4 * e], scale), __fdiv_rn(f[4 * e + 1], scale), __fdiv_rn(f[4 * e + 2], scale), __fdiv_rn(f[4 * e + 3], scale)));
-      o[e] = *reinterpret_cast<const uint32_t*>(&p4);
-    }
-    *reinterpret_cast<uint2*>(q + (size_t)row * ldq + (size_t)kb * 128 + sub * 8) = make_uint2(o[0], o[1]);
+    float f[8], unused = 0.f;
+    unpackBf16x8(raw[i], f, unused);
+    *reinterpret_cast<uint2*>(q + (size_t)row * ldq + (size_t)kb * 128 + sub * 8) = qs.codes(f);
   }
 }
 
@@ -107,6 +91,9 @@ __global__ void __launch_bounds__(256) quantBlocks128x128(const __nv_bfloat16* w
 }  // namespace b200
 
 using namespace b200;
+
+static int gemmFp8BlockTn(const void* A8, const float* sA, const void* B8, const float* sB, void* C, int M, int N, int K, int lda, int ldb, int ldc, int maxCtas,
+                          bool early, cudaStream_t st);
 
 extern "C" {
 
@@ -116,7 +103,7 @@ extern "C" {
 int b200ops_quant_e4m3_1x128_strided(const void* x, void* q, float* s, int M, int K, int ldx, int ldq, int lds, cudaStream_t st) {
   if (M <= 0 || K <= 0) return 0;
   if ((K & 127) || (ldx & 7) || (ldq & 7) || lds < M || ((uintptr_t)x & 15) || ((uintptr_t)q & 7)) return (int)cudaErrorInvalidValue;
-  gemm8::quantRows1x128<<<(M + 7) / 8, 256, 0, st>>>((const __nv_bfloat16*)x, (uint8_t*)q, s, M, K, ldx, ldq, lds);
+  gemm8::quantRows1x128<<<dim3((M + 7) / 8, (K + 256 * gemm8::kQuantRounds - 1) / (256 * gemm8::kQuantRounds)), 256, 0, st>>>((const __nv_bfloat16*)x, (uint8_t*)q, s, M, K, ldx, ldq, lds);
   return (int)cudaGetLastError();
 }
 int b200ops_quant_e4m3_1x128(const void* x, void* q, float* s, int M, int K, int ldx, int ldq, cudaStream_t st) {
@@ -135,8 +122,25 @@ int b200ops_quant_e4m3_128x128(const void* w, void* q, float* s, int N, int K, i
 // C[M, N] (bf16, ldc) = block-scaled A8[M, K] (lda bytes) * B8[N, K]^T (ldb bytes); sA [K / 128][M], sB [ceil(N / 128)][K / 128].
 int b200ops_gemm_fp8_block_tn(const void* A8, const float* sA, const void* B8, const float* sB, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                               int maxCtas, cudaStream_t st) {
+  return gemmFp8BlockTn(A8, sA, B8, sB, C, M, N, K, lda, ldb, ldc, maxCtas, false, st);
+}
+
+// C[M, N] (bf16, row stride N) = x[M, K] (bf16, row stride ldx) * B8[N, K]^T with x quantised on the way; `scratch` holds the codes and
+// behind them the scales: M * K + M * (K / 128) * 4 bytes, 16-byte aligned.
+int b200ops_fp8_linear(const void* x, void* scratch, const void* B8, const float* sB, void* C, int M, int N, int K, int ldx, int ldb, cudaStream_t st) {
+  float* s = reinterpret_cast<float*>((uint8_t*)scratch + (size_t)M * K);
+  const int e = b200ops_quant_e4m3_1x128(x, scratch, s, M, K, ldx, K, st);
+  return e ? e : gemmFp8BlockTn(scratch, s, B8, sB, C, M, N, K, K, ldb, N, 0, true, st);
+}
+
+}  // extern "C"
+
+static int gemmFp8BlockTn(const void* A8, const float* sA, const void* B8, const float* sB, void* C, int M, int N, int K, int lda, int ldb, int ldc, int maxCtas,
+                          bool early, cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((K & 127) || ((uintptr_t)C & 15) || (ldc & 7)) return (int)cudaErrorInvalidValue;
+  if (maxCtas == 0 && gemmn8::prefersNarrow(M, N, K))
+    return (int)gemmn8::gemmNarrowFp8(A8, sA, (size_t)M, 1, B8, sB, C, M, N, K, lda, ldb, ldc, false, early, st);
   gemm8::Params p{};
   if (!gemm::makeTileMap(&p.mapA, A8, M, K, lda, gemm::BM, 1) || !gemm::makeTileMap(&p.mapB, B8, N, K, ldb, gemm8::BN, 1)) return (int)cudaErrorInvalidValue;
   p.sA = sA;
@@ -166,5 +170,3 @@ int b200ops_gemm_fp8_block_tn(const void* A8, const float* sA, const void* B8, c
   gemm8::gemmFp8BlockKernel<<<ctas, gemm8::kThreads, gemm8::kSmemBytes, st>>>(p);
   return (int)cudaGetLastError();
 }
-
-}  // extern "C"

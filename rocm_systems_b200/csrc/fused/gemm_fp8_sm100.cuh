@@ -63,6 +63,46 @@ struct Params {
   int* err;          // device word: 0, or the code of the first wait that gave up (gemm::ErrCode)
 };
 
+// x / scale for the quantisers, correctly rounded like the IEEE division of the PyTorch oracles but three operations instead of a
+// division per element: with r = RN(1 / scale) and q0 = RN(x r), q = RN(q0 + r (x - q0 scale)) is the correctly rounded quotient
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990, theorem on division with a
+// correctly rounded reciprocal) as long as nothing underflows: the scale is at least 1e-10 / 448, so a quotient that does not round
+// to the code 0 has a remainder far above the smallest normal number. A scale that is not finite takes the division itself.
+struct QuantScale {
+  float scale, recip;
+  bool finite;
+  __device__ __forceinline__ explicit QuantScale(float amax) {
+    scale = fmaxf(amax, 1e-10f) * (1.f / 448.f);
+    recip = __frcp_rn(scale);
+    finite = scale <= 3.402823466e38f;
+  }
+  __device__ __forceinline__ float div(float x) const {
+    if (!finite) return __fdiv_rn(x, scale);
+    const float q = x * recip;
+    return fmaf(fmaf(-q, scale, x), recip, q);
+  }
+  // 8 bf16 values -> 8 codes
+  __device__ __forceinline__ uint2 codes(const float (&f)[8]) const {
+    uint32_t w[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const __nv_fp8x4_e4m3 p4(make_float4(div(f[4 * i]), div(f[4 * i + 1]), div(f[4 * i + 2]), div(f[4 * i + 3])));
+      w[i] = *reinterpret_cast<const uint32_t*>(&p4);
+    }
+    return make_uint2(w[0], w[1]);
+  }
+};
+__device__ __forceinline__ void unpackBf16x8(const uint4& raw, float (&f)[8], float& amax) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float2 p = __bfloat1622float2(h[i]);
+    f[2 * i] = p.x;
+    f[2 * i + 1] = p.y;
+    amax = fmaxf(amax, fmaxf(fabsf(p.x), fabsf(p.y)));
+  }
+}
+
 // Output column of accumulator element i of an epilogue thread whose warp is member h of its pair.
 __device__ __forceinline__ int accCol(int i, int h) { return (i < 32 ? 0 : 64) + h * 32 + (i & 31); }
 

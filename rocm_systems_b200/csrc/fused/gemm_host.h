@@ -23,4 +23,9 @@ namespace gemmn {
 bool prefersNarrow(int M, int N);
 cudaError_t gemmNarrowBf16(const void* X, const void* W, void* C, int M, int N, int K, int ldx, int ldw, int ldc, bool wMn, int gateUpTile, cudaStream_t s);
 }  // namespace gemmn
+namespace gemmn8 {
+bool prefersNarrow(int M, int N, int K);
+cudaError_t gemmNarrowFp8(const void* X8, const float* sX, size_t sXBlock, size_t sXRow, const void* W8, const float* sW, void* C, int M, int N, int K, int ldx,
+                          int ldw, int ldc, bool swiglu, bool early, cudaStream_t s);
+}  // namespace gemmn8
 }  // namespace b200

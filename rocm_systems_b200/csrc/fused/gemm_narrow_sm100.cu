@@ -10,7 +10,7 @@ namespace gemmn {
 namespace {
 
 template <int TN, bool W_MN, bool SWIGLU>
-cudaError_t launch(const Params& p, int tiles, int S, cudaStream_t s) {
+cudaError_t launch(const Params& p, int tiles, int groups, int S, cudaStream_t s) {
   auto kernel = gemmNarrowKernel<TN, W_MN, SWIGLU>;
   static bool configured[64] = {};
   int dev = 0;
@@ -22,7 +22,7 @@ cudaError_t launch(const Params& p, int tiles, int S, cudaStream_t s) {
     configured[dev] = true;
   }
   cudaLaunchConfig_t q{};
-  q.gridDim = dim3((unsigned)(S * tiles), (unsigned)((p.M + TN - 1) / TN));
+  q.gridDim = dim3((unsigned)(S * tiles), (unsigned)((p.M + TN - 1) / TN), (unsigned)groups);
   q.blockDim = dim3(kThreads);
   q.dynamicSmemBytes = Cfg<TN>::kSmemBytes;
   q.stream = s;
@@ -37,12 +37,12 @@ cudaError_t launch(const Params& p, int tiles, int S, cudaStream_t s) {
 }
 
 template <bool W_MN, bool SWIGLU>
-cudaError_t dispatch(const Params& p, int tn, int tiles, int S, cudaStream_t s) {
+cudaError_t dispatch(const Params& p, int tn, int tiles, int groups, int S, cudaStream_t s) {
   switch (tn) {
-    case 16: return launch<16, W_MN, SWIGLU>(p, tiles, S, s);
-    case 32: return launch<32, W_MN, SWIGLU>(p, tiles, S, s);
-    case 64: return launch<64, W_MN, SWIGLU>(p, tiles, S, s);
-    default: return launch<128, W_MN, SWIGLU>(p, tiles, S, s);
+    case 16: return launch<16, W_MN, SWIGLU>(p, tiles, groups, S, s);
+    case 32: return launch<32, W_MN, SWIGLU>(p, tiles, groups, S, s);
+    case 64: return launch<64, W_MN, SWIGLU>(p, tiles, groups, S, s);
+    default: return launch<128, W_MN, SWIGLU>(p, tiles, groups, S, s);
   }
 }
 
@@ -59,28 +59,40 @@ bool prefersNarrow(int M, int N) {
   return M <= 512 && 2 * tiles <= gemm2::pairsOnDevice();
 }
 
-// C [M, N or N / 2] = X [M, K] * W [N, K]^T; wMn: W is stored [K, N]. gateUpTile != 0: SwiGLU over the interleaved rows of W.
+// CTAs along K: as many as fill the device two to an SM. 4096 x 4096 on 16 rows takes 14.8 us with 2 splits, 10.8 - 11.4 with 4 - 8.
+// One token tile: at most 240 CTAs, because from 128 feature tiles up the exchange costs more than the second CTA of an SM gives
+// (16384 x 2048 on 16 rows: 15.2 us unsplit, 16.1 in two). A cluster beyond that number waits for a second wave (6144 x 4096: 13.5 us
+// with 240 CTAs, 18.6 with 288).
+int splitsFor(int tiles, int tokTiles, int kSteps) {
+  return std::max(1, std::min({kMaxSplit, kSteps, (tokTiles == 1 ? 240 : 256) / (tiles * tokTiles)}));
+}
+
+namespace {
+
+cudaError_t run(Params& p, const void* X, const void* W, int xRows, int groups, int tn, int ldx, int ldw, bool wMn, cudaStream_t s) {
+  const bool okW = wMn ? gemm::makeTileMap(&p.mapW, W, p.K, p.N, ldw, 64, 2) : gemm::makeTileMap(&p.mapW, W, (uint64_t)groups * p.N, p.K, ldw, 64, 2);
+  if (!okW || !gemm::makeTileMap(&p.mapX, X, xRows, p.K, ldx, tn, 2)) return cudaErrorInvalidValue;
+  p.err = gemm::errWord();
+  if (!p.err) return cudaErrorMemoryAllocation;
+  const int tiles = (p.N + BF - 1) / BF, tokTiles = groups > 1 ? 1 : (p.M + tn - 1) / tn;
+  const int S = splitsFor(tiles * groups, tokTiles, (p.K + BK - 1) / BK);
+  if (p.gateUpTile) return dispatch<false, true>(p, tn, tiles, groups, S, s);
+  return wMn ? dispatch<true, false>(p, tn, tiles, groups, S, s) : dispatch<false, false>(p, tn, tiles, groups, S, s);
+}
+
+}  // namespace
+
+// C [M, N or N / 2] = X [M, K] * W [N, K]^T; wMn: W is stored [K, N]. gateUpTile != 0: SwiGLU over the interleaved rows of W (K-major).
 cudaError_t gemmNarrowBf16(const void* X, const void* W, void* C, int M, int N, int K, int ldx, int ldw, int ldc, bool wMn, int gateUpTile, cudaStream_t s) {
+  if (wMn && gateUpTile) return cudaErrorInvalidValue;
   Params p{};
-  const int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
-  const bool okW = wMn ? gemm::makeTileMap(&p.mapW, W, K, N, ldw, 64, 2) : gemm::makeTileMap(&p.mapW, W, N, K, ldw, 64, 2);
-  if (!okW || !gemm::makeTileMap(&p.mapX, X, M, K, ldx, tn, 2)) return cudaErrorInvalidValue;
   p.C = (__nv_bfloat16*)C;
   p.ldc = ldc;
   p.M = M;
   p.N = N;
   p.K = K;
   p.gateUpTile = gateUpTile;
-  p.err = gemm::errWord();
-  if (!p.err) return cudaErrorMemoryAllocation;
-  // Split K until the CTAs fill the device (two to an SM): 4096 x 4096 on 16 rows takes 14.8 us with 2 splits, 10.8 - 11.4 with
-  // 4 - 8. One token tile: at most 240 CTAs, because from 128 feature tiles up the exchange costs more than the second CTA of an
-  // SM gives (16384 x 2048 on 16 rows: 15.2 us unsplit, 16.1 in two). A cluster beyond that number waits for a second wave
-  // (6144 x 4096: 13.5 us with 240 CTAs, 18.6 with 288).
-  const int tiles = (N + BF - 1) / BF, tokTiles = (M + tn - 1) / tn, kIters = (K + BK - 1) / BK;
-  const int S = std::max(1, std::min({kMaxSplit, kIters, (tokTiles == 1 ? 240 : 256) / (tiles * tokTiles)}));
-  if (gateUpTile) return wMn ? cudaErrorInvalidValue : dispatch<false, true>(p, tn, tiles, S, s);
-  return wMn ? dispatch<true, false>(p, tn, tiles, S, s) : dispatch<false, false>(p, tn, tiles, S, s);
+  return run(p, X, W, M, 1, M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128, ldx, ldw, wMn, s);
 }
 
 }  // namespace gemmn

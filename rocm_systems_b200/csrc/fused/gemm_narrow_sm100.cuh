@@ -42,13 +42,21 @@ template <int TN> struct Cfg {
   static_assert((size_t)TN * BF * 4 <= (size_t)kStages * kStageBytes, "the partial tile reuses the ring");
 };
 
+// Grouped form (the experts of a mixture): blockIdx.z is the group g, which owns rows [g * cap, g * cap + count[g]) of X and C and
+// rows [g * N, (g + 1) * N) of W. count == nullptr: one group of all M rows.
+struct Group {
+  const uint32_t* count;
+  int cap;
+};
+
 struct Params {
-  CUtensorMap mapW;  // K-major: [N, K], box {64, 64}. MN-major: [K, N], box {64, 64}
+  CUtensorMap mapW;  // K-major: [groups * N, K], box {64, 64}. MN-major: [K, N], box {64, 64}
   CUtensorMap mapX;  // [M, K], box {64, TN}
   __nv_bfloat16* C;
   int ldc;
-  int M, N, K;      // N: rows of W
+  int M, N, K;      // M: rows of X of the one group, N: rows of W per group
   int gateUpTile;   // SWIGLU: rows of W per interleaved block (half gate, half up)
+  Group group;
   int* err;
 };
 
@@ -58,7 +66,57 @@ __device__ __forceinline__ float4 ldSharedCluster4(uint32_t addr) {
   return v;
 }
 
-// Grid: x = split rank + S * feature tile, y = token tile; cluster (S, 1, 1).
+// Every CTA of the cluster has parked its partial tile, `part` [TN tokens][128 features] fp32, in its shared memory: this CTA adds
+// up its share of the tile's pieces of 4 output features over the S partials, in the order of K, and stores them as bf16.
+// C: the tile's first token row, n0: its first output feature, nOut: output features there are.
+template <bool SWIGLU>
+__device__ __forceinline__ void sumSplitsAndStore(const float* part, int S, int split, int tokens, __nv_bfloat16* C, int ldc, int n0, int nOut) {
+  constexpr int kPerTok = (SWIGLU ? BF / 2 : BF) / 4;
+  const int pieces = tokens * kPerTok;
+  const int lo = (int)((long long)pieces * split / S), hi = (int)((long long)pieces * (split + 1) / S);
+  const uint32_t base = sm100::smemAddr(part);
+  auto sum4 = [&](int at) {  // `at`: float index into the partial tiles
+    float4 v = *reinterpret_cast<const float4*>(part + at);
+    if (S > 1) {
+      v = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int s = 0; s < S; s++) {
+        const float4 a = ldSharedCluster4(sm100::mapToCta(base + (uint32_t)at * 4, (uint32_t)s));
+        v.x += a.x;
+        v.y += a.y;
+        v.z += a.z;
+        v.w += a.w;
+      }
+    }
+    return v;
+  };
+  for (int i = lo + (int)threadIdx.x; i < hi; i += kThreads) {
+    const int tok = i / kPerTok, f = (i % kPerTok) * 4;
+    float4 v = sum4(tok * BF + f);
+    if constexpr (SWIGLU) {
+      const float4 u = sum4(tok * BF + 64 + f);
+      v.x = v.x / (1.f + __expf(-v.x)) * u.x;
+      v.y = v.y / (1.f + __expf(-v.y)) * u.y;
+      v.z = v.z / (1.f + __expf(-v.z)) * u.z;
+      v.w = v.w / (1.f + __expf(-v.w)) * u.w;
+    }
+    const int n = n0 + f;
+    if (n >= nOut) continue;
+    __nv_bfloat16* dst = C + (size_t)tok * ldc + n;
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    if (n + 4 <= nOut) {
+      uint2 o;
+      o.x = *reinterpret_cast<const uint32_t*>(&a);
+      o.y = *reinterpret_cast<const uint32_t*>(&b);
+      *reinterpret_cast<uint2*>(dst) = o;
+    } else {
+      dst[0] = a.x;
+      if (n + 1 < nOut) dst[1] = a.y;
+      if (n + 2 < nOut) dst[2] = b.x;
+    }
+  }
+}
+
+// Grid: x = split rank + S * feature tile, y = token tile, z = group; cluster (S, 1, 1).
 template <int TN, bool W_MN, bool SWIGLU>
 __global__ void __launch_bounds__(kThreads, 2) gemmNarrowKernel(const __grid_constant__ Params p, int S) {
   using C = Cfg<TN>;
@@ -87,7 +145,12 @@ __global__ void __launch_bounds__(kThreads, 2) gemmNarrowKernel(const __grid_con
     row0 = n0 / half * p.gateUpTile + n0 % half;
     row1 = row0 + half;
   }
+  row0 += (int)blockIdx.z * p.N;
+  row1 += (int)blockIdx.z * p.N;
   const int tok0 = blockIdx.y * TN;
+  const int xRow0 = (int)blockIdx.z * p.group.cap;
+  const int rows = p.group.count ? min((int)p.group.count[blockIdx.z], p.group.cap) : p.M;
+  if (tok0 >= rows) return;  // the same for the whole cluster
   const int kAll = (p.K + BK - 1) / BK;
   const int k0 = (int)((long long)kAll * split / S), k1 = (int)((long long)kAll * (split + 1) / S);
 
@@ -125,7 +188,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemmNarrowKernel(const __grid_con
           if constexpr (W_MN) tmaLoad2d(sw + h * kHalfBytes, &p.mapW, row, k * BK, &full[stage]);
           else tmaLoad2d(sw + h * kHalfBytes, &p.mapW, k * BK, row, &full[stage]);
         }
-        tmaLoad2d(smemX + (size_t)stage * C::kXBytes, &p.mapX, k * BK, tok0, &full[stage]);
+        tmaLoad2d(smemX + (size_t)stage * C::kXBytes, &p.mapX, k * BK, xRow0 + tok0, &full[stage]);
         if (++stage == C::kStages) { stage = 0; phase ^= 1; }
       }
       if (!ok)
@@ -180,53 +243,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemmNarrowKernel(const __grid_con
   } else {
     __syncthreads();
   }
-  // Sum over the splits: this CTA's share of the tile's pieces of 4 output features.
-  {
-    constexpr int kPerTok = kOut / 4;
-    const int nOut = SWIGLU ? p.N / 2 : p.N;
-    const int pieces = min(TN, p.M - tok0) * kPerTok;
-    const int lo = (int)((long long)pieces * split / S), hi = (int)((long long)pieces * (split + 1) / S);
-    const uint32_t base = smemAddr(part);
-    auto sum4 = [&](int at) {  // `at`: float index into the partial tiles
-      float4 v = *reinterpret_cast<const float4*>(part + at);
-      if (S > 1) {
-        v = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s = 0; s < S; s++) {
-          const float4 a = ldSharedCluster4(mapToCta(base + (uint32_t)at * 4, (uint32_t)s));
-          v.x += a.x;
-          v.y += a.y;
-          v.z += a.z;
-          v.w += a.w;
-        }
-      }
-      return v;
-    };
-    for (int i = lo + (int)threadIdx.x; i < hi; i += kThreads) {
-      const int tok = i / kPerTok, f = (i % kPerTok) * 4;
-      float4 v = sum4(tok * BF + f);
-      if constexpr (SWIGLU) {
-        const float4 u = sum4(tok * BF + 64 + f);
-        v.x = v.x / (1.f + __expf(-v.x)) * u.x;
-        v.y = v.y / (1.f + __expf(-v.y)) * u.y;
-        v.z = v.z / (1.f + __expf(-v.z)) * u.z;
-        v.w = v.w / (1.f + __expf(-v.w)) * u.w;
-      }
-      const int n = n0 + f;
-      if (n >= nOut) continue;
-      __nv_bfloat16* dst = p.C + (size_t)(tok0 + tok) * p.ldc + n;
-      const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-      if (n + 4 <= nOut) {
-        uint2 o;
-        o.x = *reinterpret_cast<const uint32_t*>(&a);
-        o.y = *reinterpret_cast<const uint32_t*>(&b);
-        *reinterpret_cast<uint2*>(dst) = o;
-      } else {
-        dst[0] = a.x;
-        if (n + 1 < nOut) dst[1] = a.y;
-        if (n + 2 < nOut) dst[2] = b.x;
-      }
-    }
-  }
+  sumSplitsAndStore<SWIGLU>(part, S, split, min(TN, rows - tok0), p.C + (size_t)(xRow0 + tok0) * p.ldc, p.ldc, n0, SWIGLU ? p.N / 2 : p.N);
   if (S > 1) {
     clusterArrive();  // no CTA leaves while a peer still reads its partial tile
     clusterWait();

@@ -56,6 +56,12 @@ __device__ __forceinline__ bool mbarWait(uint64_t* bar, uint32_t parity, volatil
   return false;
 }
 
+// ---- programmatic dependent launch ------------------------------------------------------------------
+// Lets the next kernel of the stream, if it was launched with programmatic stream serialisation, start before this one ends.
+__device__ __forceinline__ void gridLaunchDependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Until the kernels in front have ended and their writes are visible; returns at once in a kernel launched without the attribute.
+__device__ __forceinline__ void gridDependencyWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- TMA ------------------------------------------------------------------------------------------
 // 2-D tile load, global -> shared, completion counted in bytes on `bar`. x is the innermost
 // coordinate (elements) and must keep x * sizeof(element) a multiple of 16 bytes.

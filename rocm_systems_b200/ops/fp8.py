@@ -78,6 +78,7 @@ def _lib():
         lib.b200ops_quant_e4m3_1x128.argtypes = [vp, vp, vp, i32, i32, i32, i32, vp]
         lib.b200ops_quant_e4m3_1x128_strided.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, vp]
         lib.b200ops_quant_e4m3_128x128.argtypes = [vp, vp, vp, i32, i32, i32, i32, vp]
+        lib.b200ops_fp8_linear.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]
         lib.b200ops_gemm_fp8_block_tn.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp]
         lib._fp8_sig = True
     return lib
@@ -129,5 +130,14 @@ def gemm(xq: torch.Tensor, xs: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor,
 
 def linear(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor) -> torch.Tensor:
     """``x @ w.T`` for bf16 ``x`` against a weight quantised once with ``quantize_weight``."""
-    xq, xs = quantize_act(x)
-    return gemm(xq, xs, wq, ws)
+    assert x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] % 128 == 0
+    assert wq.dtype == torch.float8_e4m3fn and wq.stride(1) == 1 and wq.shape[1] == x.shape[1]
+    M, K = x.shape
+    N = wq.shape[0]
+    assert tuple(ws.shape) == ((N + 127) // 128, K // 128) and ws.is_contiguous()
+    scratch = torch.empty(M * K + M * (K // 32), dtype=torch.uint8, device=x.device)   # codes, then 4 bytes of scale per 128 of them
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
+    train_ops._ck(_lib().b200ops_fp8_linear(x.data_ptr(), scratch.data_ptr(), wq.data_ptr(), ws.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), wq.stride(0),
+                                            train_ops._s()), "fp8_linear")
+    train_ops.LAUNCHES += 1
+    return out

@@ -78,3 +78,42 @@ def test_gemm_of_few_rows_matches_fp32(M, N, K, wt):
     err = (big[:M, :N].double() - ref).abs()
     assert bool((err <= ref.abs() * 2.0 ** -8 + 6 / 16 * K ** 1.5 * 2.0 ** -23).all()), float((err - ref.abs() * 2.0 ** -8).max())
     assert bool((big[M:] == 7).all()) and bool((big[:, N:] == 7).all())     # nothing outside the view was written
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (1, 1000, 256), (16, 6144, 4096), (17, 136, 384), (32, 4096, 14336), (33, 4096, 1152), (64, 28672, 512),
+                                   (65, 1032, 640), (128, 264, 4096), (192, 512, 8192), (257, 640, 384), (16, 136, 16512)])
+def test_fp8_linear_of_few_rows_matches_the_oracle(M, N, K):
+    """The block-scaled kernel with output features as MMA rows (one to four token tiles, ragged edges, more splits than blocks of K, a K
+    whose scales just do not fit), behind the quantiser it may overlap. Products of codes are exact in fp32; bound: the bf16 rounding of
+    the result and one fp32 rounding per block and split of a sum that stays below the sum of magnitudes."""
+    from rocm_systems_b200.ops import fp8
+    from rocm_systems_b200.ops import train_ops as ops
+
+    torch.manual_seed(M + N + K)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    wq, ws = fp8.quantize_weight((torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16))
+    xq, xs = fp8.quantize_act(x)
+    rq, rs = fp8.ref_quantize_act(x)
+    assert torch.equal(xq.view(torch.uint8), rq.view(torch.uint8)) and torch.equal(xs, rs)
+    a, b = fp8.ref_dequantize_act(xq, xs).double(), fp8.ref_dequantize_weight(wq, ws).double()
+    ref = a @ b.t()
+    tol = ref.abs() * 2.0 ** -8 + (a.abs() @ b.abs().t()) * 2.0 ** -24 * (K // 128 + 16)
+    for out in (fp8.linear(x, wq, ws), fp8.gemm(xq, xs, wq, ws)):
+        torch.cuda.synchronize()
+        assert ops.gemm_take_error() == 0
+        assert bool(((out.double() - ref).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("size", [1e-30, 1e-12, 1.0, 1e30])
+def test_quantiser_codes_are_those_of_an_ieee_division(size):
+    """Every bf16 significand over scales drawn from the data: codes and scales of both quantisers are bit-equal to the oracles', which divide."""
+    from rocm_systems_b200.ops import fp8
+
+    torch.manual_seed(1)
+    x = (torch.randn(1500, 2176, device="cuda") * size).to(torch.bfloat16)
+    x[0, :128] = 0
+    x[1, 3] = float("inf")
+    for got, want in ((fp8.quantize_act(x), fp8.ref_quantize_act(x)), (fp8.quantize_weight(x[2:]), fp8.ref_quantize_weight(x[2:]))):
+        assert torch.equal(got[0].view(torch.uint8) & 0x7f == 0x7f, want[0].view(torch.uint8) & 0x7f == 0x7f)   # NaN (inf / inf) in the same places
+        ok = want[0].view(torch.uint8) & 0x7f != 0x7f
+        assert torch.equal(got[0].view(torch.uint8)[ok], want[0].view(torch.uint8)[ok]) and torch.equal(got[1], want[1])
