@@ -41,7 +41,7 @@ def _lib_ops():
 
 
 def _s() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ck(rc: int, what: str) -> None:
