@@ -141,6 +141,8 @@ static int gemmFp8BlockTn(const void* A8, const float* sA, const void* B8, const
   if ((K & 127) || ((uintptr_t)C & 15) || (ldc & 7)) return (int)cudaErrorInvalidValue;
   if (maxCtas == 0 && gemmn8::prefersNarrow(M, N, K))
     return (int)gemmn8::gemmNarrowFp8(A8, sA, (size_t)M, 1, B8, sB, C, M, N, K, lda, ldb, ldc, false, early, st);
+  if (maxCtas == 0 && gemm8p::prefersPair(M, N, K))
+    return (int)gemm8p::gemmFp8Pair(A8, sA, (size_t)M, 1, B8, sB, C, M, N, K, lda, ldb, ldc, false, st);
   gemm8::Params p{};
   if (!gemm::makeTileMap(&p.mapA, A8, M, K, lda, gemm::BM, 1) || !gemm::makeTileMap(&p.mapB, B8, N, K, ldb, gemm8::BN, 1)) return (int)cudaErrorInvalidValue;
   p.sA = sA;

@@ -70,16 +70,14 @@ struct Params {
 // to the code 0 has a remainder far above the smallest normal number. A scale that is not finite takes the division itself.
 struct QuantScale {
   float scale, recip;
-  bool finite;
   __device__ __forceinline__ explicit QuantScale(float amax) {
     scale = fmaxf(amax, 1e-10f) * (1.f / 448.f);
     recip = __frcp_rn(scale);
-    finite = scale <= 3.402823466e38f;
   }
   __device__ __forceinline__ float div(float x) const {
-    if (!finite) return __fdiv_rn(x, scale);
     const float q = x * recip;
-    return fmaf(fmaf(-q, scale, x), recip, q);
+    const float r = fmaf(fmaf(-q, scale, x), recip, q);
+    return recip != 0.f ? r : __fdiv_rn(x, scale);
   }
   // 8 bf16 values -> 8 codes
   __device__ __forceinline__ uint2 codes(const float (&f)[8]) const {

@@ -56,6 +56,10 @@ __device__ __forceinline__ bool mbarWait(uint64_t* bar, uint32_t parity, volatil
   return false;
 }
 
+// ---- registers of a warpgroup (every warp of it executes these; the shares of a CTA add up to at most what it was launched with) ----
+template <int N> __device__ __forceinline__ void setMaxRegsUp() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void setMaxRegsDown() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // ---- programmatic dependent launch ------------------------------------------------------------------
 // Lets the next kernel of the stream, if it was launched with programmatic stream serialisation, start before this one ends.
 __device__ __forceinline__ void gridLaunchDependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -175,8 +179,10 @@ __device__ __forceinline__ uint32_t mapToCta(uint32_t smemByteAddr, uint32_t ran
 }
 __device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Arrive on a barrier of any CTA of the cluster. What it orders are tensor-memory accesses, through the tcgen05 fences on both sides,
+// and no memory writes: the default release at CTA scope, as a cluster-scope release waits several hundred cycles for nothing.
 __device__ __forceinline__ void mbarArriveCluster(uint32_t clusterAddr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(clusterAddr) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(clusterAddr) : "memory");
 }
 // Tile load into THIS CTA's shared memory whose bytes are counted on a barrier of the pair's even CTA (`barClusterAddr`).
 __device__ __forceinline__ void tmaLoad2dPair(void* smemDst, const CUtensorMap* map, int x, int y, uint32_t barClusterAddr) {
@@ -196,6 +202,14 @@ __device__ __forceinline__ void mmaF16Pair(uint32_t tmemD, uint64_t descA, uint6
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmemD),
+      "l"(descA), "l"(descB), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mmaF8Pair(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmemD),
       "l"(descA), "l"(descB), "r"(idesc), "r"(accumulate)
       : "memory");
 }

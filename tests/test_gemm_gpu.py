@@ -117,3 +117,22 @@ def test_quantiser_codes_are_those_of_an_ieee_division(size):
         assert torch.equal(got[0].view(torch.uint8) & 0x7f == 0x7f, want[0].view(torch.uint8) & 0x7f == 0x7f)   # NaN (inf / inf) in the same places
         ok = want[0].view(torch.uint8) & 0x7f != 0x7f
         assert torch.equal(got[0].view(torch.uint8)[ok], want[0].view(torch.uint8)[ok]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("M,N,K", [(1000, 8200, 1152), (129, 28680, 1152), (513, 8192, 1152), (2049, 8200, 640), (4096, 6144, 512), (4097, 4104, 512)])
+def test_fp8_gemm_on_cta_pairs_equals_the_one_cta_kernel(M, N, K):
+    """Sizes that the rule sends to CTA pairs (ragged rows, columns and an odd number of blocks of K): every partial product is folded in the
+    same order with the same operations, so the results are bit-equal to the kernel that a CTA limit asks for. Strided output; nothing else is written."""
+    from rocm_systems_b200.ops import fp8
+    from rocm_systems_b200.ops import train_ops as ops
+
+    torch.manual_seed(M + N + K)
+    xq, xs = fp8.quantize_act(torch.randn(M, K, device="cuda").to(torch.bfloat16))
+    wq, ws = fp8.quantize_weight((torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16))
+    big = torch.full((M + 1, N + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    fp8.gemm(xq, xs, wq, ws, out=big[:M, :N])
+    want = fp8.gemm(xq, xs, wq, ws, max_ctas=148)
+    torch.cuda.synchronize()
+    assert ops.gemm_take_error() == 0
+    assert torch.equal(big[:M, :N], want)
+    assert bool((big[M:] == 7).all()) and bool((big[:, N:] == 7).all())
