@@ -9,9 +9,9 @@
 //               CTA 0 waits (bounded) until every peer said so, so when the kernel ends the receive
 //               buffers and the per-expert counts are complete.
 //   epDequant   fp8 rows -> bf16 rows for the grouped GEMMs.
-//   grouped GEMMs run on the tcgen05 kernel with a policy that walks a compact list of (expert, row block,
-//               column block): only row blocks that hold tokens are numbered, so the persistent CTAs share the
-//               real work evenly; the first one applies SwiGLU in its epilogue.
+//   grouped GEMMs run on the tcgen05 kernels in their grouped forms: CTA pairs walk a compact list of (row block with
+//               tokens, column block), so the persistent CTAs share the real work evenly however the tokens fell; with a few
+//               rows per expert the kernels with features as MMA rows. The first GEMM applies SwiGLU in its epilogue.
 //   epCombine   ONE kernel at the token's home rank: for each of the k experts it pulls the expert's
 //               output row from the owning rank (peer loads) and accumulates gate * row in fp32,
 //               in the fixed order k = 0..k-1, so the result is deterministic.
@@ -28,12 +28,12 @@
 #include "b200coll/fused.h"
 #include "gemm_fp8_sm100.cuh"
 #include "gemm_host.h"
-#include "gemm_sm100.cuh"
 
 namespace b200 {
 namespace ep {
 
 constexpr int kMaxTopK = 8;
+constexpr int kMaxLocalExperts = 64;
 
 // Layout of the symmetric EP window of one rank (all offsets in bytes, 256-byte aligned).
 struct EpLayout {
@@ -68,14 +68,16 @@ __host__ inline EpLayout makeLayout(int nranks, int expertsLocal, int cap, int h
 // A NaN logit counts as -inf and +inf as the largest finite value, so every id written lies in [0, E)
 // and every weight is finite: a row with fewer than k selectable values (all NaN, mostly -inf) fills up
 // with the lowest expert ids not yet taken, and a row whose selected logits are all -inf gets weights 1/k.
+// PER: a power of two, at least E / 32 (with 32 candidates per lane for any E, the 4096 rows of a 32-expert layer took 27 us).
+template <int PER>
 __global__ void __launch_bounds__(256) epRoute(const float* __restrict__ logits, int* __restrict__ topIdx, float* __restrict__ topW, int T, int E, int k) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= T) return;
   const float* row = logits + (size_t)warp * E;
-  const int per = E / 32;  // <= 32
-  float v[32];
+  const int per = E / 32;  // <= PER
+  float v[PER];
 #pragma unroll
-  for (int i = 0; i < 32; i++) {
+  for (int i = 0; i < PER; i++) {
     float x = i < per ? row[i * 32 + lane] : -INFINITY;
     x = x == x ? fminf(x, 3.402823466e38f) : -INFINITY;
     v[i] = x;
@@ -87,7 +89,7 @@ __global__ void __launch_bounds__(256) epRoute(const float* __restrict__ logits,
     float best = -INFINITY;
     int bi = 0x7fffffff;  // no candidate on this lane (all taken)
 #pragma unroll
-    for (int i = 0; i < 32; i++)
+    for (int i = 0; i < PER; i++)
       if (i < per && !((taken >> i) & 1u) && (bi == 0x7fffffff || v[i] > best)) { best = v[i]; bi = i * 32 + lane; }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -129,7 +131,7 @@ __global__ void __launch_bounds__(256) epDispatch(const __grid_constant__ Dispat
   const int lane = threadIdx.x & 31;
   const int warpsPerCta = blockDim.x >> 5;
   const int gw = blockIdx.x * warpsPerCta + (threadIdx.x >> 5), nw = gridDim.x * warpsPerCta;
-  const int H = a.L.hidden, groups = H / 128, rounds = H / 256;  // a round = 32 lanes x 8 channels
+  const int H = a.L.hidden, groups = H / 128, rounds = H / 512;  // a round = 32 lanes x 16 channels
   const int rank = c.rank;
 
   // The counters of the other parity belong to the next call: clear them now.
@@ -139,63 +141,51 @@ __global__ void __launch_bounds__(256) epDispatch(const __grid_constant__ Dispat
   }
 
   for (int t = gw; t < a.T; t += nw) {
-    // Quantise the token once: lane l holds channels (j * 32 + l) * 8 .. +8 for every round j.
-    uint2 q[28];   // up to 7168 channels
-    float sc[28];  // scale of the lane's group in round j (valid on every lane of the half-warp)
+    // Lane r reserves the row of the token's r-th expert: the k atomics travel together, behind the loads of the token.
+    int e = -1, slot = -1;
     const uint4* xr = reinterpret_cast<const uint4*>(a.x + (size_t)t * H);
-#pragma unroll
-    for (int j = 0; j < 28; j++) {
-      if (j < rounds) {
-        const uint4 raw = xr[j * 32 + lane];
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-        float f[8];
-        float amax = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const float2 p = __bfloat1622float2(h[i]);
-          f[2 * i] = p.x; f[2 * i + 1] = p.y;
-          amax = fmaxf(amax, fmaxf(fabsf(p.x), fabsf(p.y)));
-        }
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));  // 16 lanes = 128 channels
-        const float scale = fmaxf(amax, 1e-10f) * (1.f / 448.f);
-            sc[j] = scale;
-        uint32_t w[2];
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-          const __nv_fp8x4_e4m3 p4(make_float4(__fdiv_rn(f[4 * i], scale), __fdiv_rn(f[4 * i + 1], scale), __fdiv_rn(f[4 * i + 2], scale), __fdiv_rn(f[4 * i + 3], scale)));
-          w[i] = *reinterpret_cast<const uint32_t*>(&p4);
-        }
-        q[j] = make_uint2(w[0], w[1]);
-      }
-    }
-    for (int r = 0; r < a.k; r++) {
-      const int e = a.topIdx[(size_t)t * a.k + r];
+    if (lane < a.k) {
+      e = a.topIdx[(size_t)t * a.k + lane];
       if (e < 0 || e >= a.L.nranks * a.L.expertsLocal) {  // not an expert: counted like a row that found its expert full, no window touched
-        if (lane == 0) {
-          atomicAdd(a.dropped, 1);
-          a.sentSlot[(size_t)t * a.k + r] = -1;
-        }
-        continue;
-      }
-      const int dst = e / a.L.expertsLocal, el = e - dst * a.L.expertsLocal;
-      int slot = 0;
-      if (lane == 0) {
+        atomicAdd(a.dropped, 1);
+      } else {
+        const int dst = e / a.L.expertsLocal, el = e - dst * a.L.expertsLocal;
         uint32_t* cnt = (uint32_t*)(a.win[dst] + a.L.cntOff) + (size_t)a.parity * a.L.expertsLocal + el;
         asm volatile("atom.relaxed.sys.global.add.u32 %0, [%1], 1;" : "=r"(slot) : "l"(cnt) : "memory");
         if (slot >= a.L.cap) { slot = -1; atomicAdd(a.dropped, 1); }
-        a.sentSlot[(size_t)t * a.k + r] = slot;
       }
-      slot = __shfl_sync(0xffffffffu, slot, 0);
-      if (slot < 0) continue;
-      const size_t rowIdx = (size_t)el * a.L.cap + slot;
-      uint2* pay = reinterpret_cast<uint2*>(a.win[dst] + a.L.payloadOff + rowIdx * H);
+      a.sentSlot[(size_t)t * a.k + lane] = slot;
+    }
+    // Quantise the token once: lane l holds channels (j * 32 + l) * 16 .. +16 of every round j, eight lanes are one group of 128.
+    uint4 q[14];   // up to 7168 channels
+    float sc[14];
+#pragma unroll
+    for (int j = 0; j < 14; j++) {
+      if (j < rounds) {
+        const uint4 r0 = xr[(j * 32 + lane) * 2], r1 = xr[(j * 32 + lane) * 2 + 1];
+        float f0[8], f1[8], amax = 0.f;
+        gemm8::unpackBf16x8(r0, f0, amax);
+        gemm8::unpackBf16x8(r1, f1, amax);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        const gemm8::QuantScale qs(amax);
+        sc[j] = qs.scale;
+        const uint2 c0 = qs.codes(f0), c1 = qs.codes(f1);
+        q[j] = make_uint4(c0.x, c0.y, c1.x, c1.y);
+      }
+    }
+    for (int r = 0; r < a.k; r++) {
+      const int sr = __shfl_sync(0xffffffffu, slot, r), er = __shfl_sync(0xffffffffu, e, r);
+      if (sr < 0) continue;
+      const int dst = er / a.L.expertsLocal, el = er - dst * a.L.expertsLocal;
+      const size_t rowIdx = (size_t)el * a.L.cap + sr;
+      uint4* pay = reinterpret_cast<uint4*>(a.win[dst] + a.L.payloadOff + rowIdx * H);
       float* scl = reinterpret_cast<float*>(a.win[dst] + a.L.scaleOff) + rowIdx * groups;
 #pragma unroll
-      for (int j = 0; j < 28; j++) {
+      for (int j = 0; j < 14; j++) {
         if (j < rounds) {
           pay[j * 32 + lane] = q[j];
-          if ((lane & 15) == 0) scl[j * 2 + (lane >> 4)] = sc[j];
+          if ((lane & 7) == 0) scl[j * 4 + (lane >> 3)] = sc[j];
         }
       }
       if (lane == 0) reinterpret_cast<int2*>(a.win[dst] + a.L.metaOff)[rowIdx] = make_int2(rank, t * kMaxTopK + r);
@@ -239,153 +229,28 @@ __global__ void __launch_bounds__(256) epDequant(const char* __restrict__ win, E
     const uint2* pay = reinterpret_cast<const uint2*>(win + L.payloadOff + (size_t)rowIdx * H);
     const float* scl = reinterpret_cast<const float*>(win + L.scaleOff) + (size_t)rowIdx * groups;
     uint4* dst = reinterpret_cast<uint4*>(xb + (size_t)rowIdx * H);
-    for (int j = 0; j < rounds; j++) {
-      const uint2 q = pay[j * 32 + lane];
-      const float s = scl[j * 2 + (lane >> 4)];
-      const __nv_fp8x4_e4m3* p4 = reinterpret_cast<const __nv_fp8x4_e4m3*>(&q);
-      const float4 lo = float4(p4[0]), hi = float4(p4[1]);
-      uint4 o;
-      __nv_bfloat162 h0 = __floats2bfloat162_rn(lo.x * s, lo.y * s), h1 = __floats2bfloat162_rn(lo.z * s, lo.w * s);
-      __nv_bfloat162 h2 = __floats2bfloat162_rn(hi.x * s, hi.y * s), h3 = __floats2bfloat162_rn(hi.z * s, hi.w * s);
-      o.x = *reinterpret_cast<uint32_t*>(&h0); o.y = *reinterpret_cast<uint32_t*>(&h1);
-      o.z = *reinterpret_cast<uint32_t*>(&h2); o.w = *reinterpret_cast<uint32_t*>(&h3);
-      dst[j * 32 + lane] = o;
-    }
-  }
-}
-
-// ---- grouped expert GEMM policy ------------------------------------------------------------------------------
-using namespace gemm;
-template <int BN, bool SWIGLU> struct GroupPolicy {
-  const uint32_t* cnt;   // rows per expert (may exceed cap when rows were dropped)
-  int experts;           // local experts
-  const int* prefix;     // shared memory, filled by the kernel: row blocks with tokens before expert e; [experts] = all of them
-  int cap, capTiles;     // rows reserved per expert, in rows and in BM-row blocks
-  int wRows;             // weight rows per expert
-  __nv_bfloat16* out;    // [expertsLocal * cap, nOut]
-  int ldo, nOut;
-  __device__ __forceinline__ int have(int e) const { return min((int)cnt[e], cap); }
-  // Tile t of the COMPACT list: only row blocks that hold tokens are numbered, expert after expert, so every CTA of the
-  // persistent grid gets the same share of real work however unevenly the tokens fell (a buffer is sized for several
-  // times the average count, so most of its row blocks are empty). Indices past the end map to no tile.
-  __device__ __forceinline__ void coord(int t, int, int tilesN, int& tm, int& tn) const {
-    const int rb = t / tilesN;
-    tn = t - rb * tilesN;
-    tm = -1;
-    if (rb >= prefix[experts]) return;
-    int e = 0;
-    while (prefix[e + 1] <= rb) e++;  // prefix[] sits in shared memory: a few cycles per step
-    tm = e * capTiles + (rb - prefix[e]);
-  }
-  __device__ __forceinline__ bool valid(int tm, int) const { return tm >= 0; }
-  __device__ __forceinline__ int aRow(int tm) const { return tm * BM; }
-  __device__ __forceinline__ int bRow(int tm, int tn) const { return (tm / capTiles) * wRows + tn * BN; }
-  __device__ __forceinline__ bool waitTile(int, int, volatile int*) const { return true; }
-  __device__ __forceinline__ void tileDone(int, int, int, int) const {}
-  __device__ __forceinline__ void drain(uint32_t taddr, int tm, int tn, int q, int lane, uint8_t* sw) const {
-    const int e = tm / capTiles;
-    const int row0 = tm * BM + q * 32;
-    const int rowsHave = have(e) - (row0 - e * cap);  // rows of this warp's 32 that hold tokens
-    if constexpr (SWIGLU) {
-      drainStaged(
-          sw, lane, BN / 2, nOut - tn * (BN / 2),
-          [&](int c, uint32_t(&g)[32]) {
-            uint32_t u[32];
-            sm100::tmemLoad32(taddr + c * 32, g);
-            sm100::tmemLoad32(taddr + BN / 2 + c * 32, u);
-            sm100::tmemLoadWait();
+    for (int j = 0; j < rounds; j += 4) {  // hidden is a multiple of 1024
+      uint2 q[4];
+      float sc[4];
 #pragma unroll
-            for (int i = 0; i < 32; i++) {
-              const float gv = __uint_as_float(g[i]);
-              g[i] = __float_as_uint(gv / (1.f + __expf(-gv)) * __uint_as_float(u[i]));
-            }
-          },
-          [&](int r) -> __nv_bfloat16* { return r < rowsHave ? out + (size_t)(row0 + r) * ldo + (size_t)tn * (BN / 2) : nullptr; });
-    } else {
-      drainStaged(
-          sw, lane, BN, nOut - tn * BN,
-          [&](int c, uint32_t(&acc)[32]) {
-            sm100::tmemLoad32(taddr + c * 32, acc);
-            sm100::tmemLoadWait();
-          },
-          [&](int r) -> __nv_bfloat16* { return r < rowsHave ? out + (size_t)(row0 + r) * ldo + (size_t)tn * BN : nullptr; });
-    }
-  }
-};
-
-// ---- first expert GEMM straight on the received fp8 rows ---------------------------------------------------------
-// The rows in the window already are what the block-scaled GEMM wants: e4m3 with one fp32 scale per row and 128
-// channels (row-major here, [row][hidden / 128]). With the experts' gate/up weight quantised per 128 x 128 block
-// (interleaved per 128 rows: 64 gate rows, then the 64 up rows of the same outputs) the dequantisation pass and its
-// bf16 copy of the activations disappear, and the larger of the two GEMMs runs at fp8 rate.
-struct GroupPolicy8 {
-  const uint32_t* cnt;  // rows per expert (may exceed cap when rows were dropped)
-  int experts;          // local experts
-  const int* prefix;    // shared memory, filled by the kernel: row blocks with tokens before expert e; [experts] = all of them
-  int cap, capTiles;
-  int wRows;            // weight rows per expert (2 ffn)
-  const float* sA;      // [expertsLocal * cap][groups]
-  int groups;           // hidden / 128
-  __nv_bfloat16* out;   // act [expertsLocal * cap, nOut]
-  int ldo, nOut;
-  __device__ __forceinline__ int have(int e) const { return min((int)cnt[e], cap); }
-  // Tile t of the COMPACT list: only row blocks that hold tokens are numbered, expert after expert, so every CTA of the
-  // persistent grid gets the same share of real work however unevenly the tokens fell (a buffer is sized for several
-  // times the average count, so most of its row blocks are empty). Indices past the end map to no tile.
-  __device__ __forceinline__ void coord(int t, int, int tilesN, int& tm, int& tn) const {
-    const int rb = t / tilesN;
-    tn = t - rb * tilesN;
-    tm = -1;
-    if (rb >= prefix[experts]) return;
-    int e = 0;
-    while (prefix[e + 1] <= rb) e++;  // prefix[] sits in shared memory: a few cycles per step
-    tm = e * capTiles + (rb - prefix[e]);
-  }
-  __device__ __forceinline__ bool valid(int tm, int) const { return tm >= 0; }
-  __device__ __forceinline__ int bRow(int tm, int tn) const { return (tm / capTiles) * wRows + tn * gemm8::BN; }
-  __device__ __forceinline__ int scaleBOff(int tm, int tn) const { return ((tm / capTiles) * (wRows / gemm8::BN) + tn) * groups; }
-  __device__ __forceinline__ bool waitTile(int, int, volatile int*) const { return true; }
-  __device__ __forceinline__ bool epiBegin(int, volatile int*) const { return true; }
-  __device__ __forceinline__ float scaleA(int kb, int row) const { return __ldg(sA + (size_t)row * groups + kb); }
-  __device__ __forceinline__ void emit(float (&acc)[gemm8::kAccCols], int tm, int tn, int q, int h, int lane, uint8_t* sw) const {
-    constexpr int H = gemm8::BN / 2;
-    const int e = tm / capTiles;
-    const int row0 = tm * gemm::BM + q * 32;
-    const int rowsHave = have(e) - (row0 - e * cap);  // rows of this warp's 32 that hold tokens
-    // gate columns 32h .. 32h+32 of the tile in acc[0..32), the up columns of the same outputs in acc[32..64)
+      for (int u = 0; u < 4; u++) {
+        q[u] = pay[(j + u) * 32 + lane];
+        sc[u] = scl[(j + u) * 2 + (lane >> 4)];
+      }
 #pragma unroll
-    for (int i = 0; i < 32; i++) {
-      const float g = acc[i];
-      acc[i] = g / (1.f + __expf(-g)) * acc[32 + i];
+      for (int u = 0; u < 4; u++) {
+        const float s = sc[u];
+        const __nv_fp8x4_e4m3* p4 = reinterpret_cast<const __nv_fp8x4_e4m3*>(&q[u]);
+        const float4 lo = float4(p4[0]), hi = float4(p4[1]);
+        uint4 o;
+        __nv_bfloat162 h0 = __floats2bfloat162_rn(lo.x * s, lo.y * s), h1 = __floats2bfloat162_rn(lo.z * s, lo.w * s);
+        __nv_bfloat162 h2 = __floats2bfloat162_rn(hi.x * s, hi.y * s), h3 = __floats2bfloat162_rn(hi.z * s, hi.w * s);
+        o.x = *reinterpret_cast<uint32_t*>(&h0); o.y = *reinterpret_cast<uint32_t*>(&h1);
+        o.z = *reinterpret_cast<uint32_t*>(&h2); o.w = *reinterpret_cast<uint32_t*>(&h3);
+        dst[(j + u) * 32 + lane] = o;
+      }
     }
-    gemm8::storeCols<32>(
-        sw, lane, H, acc,  // ffn is a multiple of 128: every tile has all of its 64 output columns
-        [&](int r) -> __nv_bfloat16* { return r < rowsHave ? out + (size_t)(row0 + r) * ldo + (size_t)tn * H : nullptr; }, [&](int) { return h * 32; });
   }
-  __device__ __forceinline__ void tileDone(int, int, int, int, int) const {}
-};
-
-constexpr int kMaxLocalExperts = 64;
-
-// Row blocks with tokens before every expert, once per CTA, into shared memory (the compact tile list of the policies).
-__device__ __forceinline__ void fillBlockPrefix(int* prefix, const uint32_t* cnt, int experts, int cap) {
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int e = 0; e < experts; e++) {
-      prefix[e] = acc;
-      acc += (min((int)cnt[e], cap) + gemm::BM - 1) / gemm::BM;
-    }
-    prefix[experts] = acc;
-  }
-  __syncthreads();
-}
-
-__global__ void __launch_bounds__(gemm8::kThreads, 1) groupedGemmFp8Kernel(const __grid_constant__ gemm8::Params p, GroupPolicy8 pol) {
-  extern __shared__ uint8_t smemRaw[];
-  __shared__ int prefix[kMaxLocalExperts + 1];
-  fillBlockPrefix(prefix, pol.cnt, pol.experts, pol.cap);
-  pol.prefix = prefix;
-  gemm8::gemmFp8Cta(p, pol, blockIdx.x, gridDim.x, smemRaw);
 }
 
 // ---- combine ---------------------------------------------------------------------------------------------------
@@ -528,36 +393,112 @@ __global__ void __launch_bounds__(256) epGatherGrad(const __grid_constant__ Gath
   const int totalRows = a.L.expertsLocal * a.L.cap;
   for (int rowIdx = gw; rowIdx < totalRows; rowIdx += nw) {
     const int e = rowIdx / a.L.cap, r = rowIdx - e * a.L.cap;
-    if (r >= min((int)cnt[e], a.L.cap)) continue;
+    const int have = min((int)cnt[e], a.L.cap);
+    if (r >= ((have + 15) & ~15)) continue;  // the weight-gradient GEMM reduces over rows in steps of 16: the last step's others are zeros
     const int2 m = meta[rowIdx];
     const int src = m.x, t = m.y / kMaxTopK, kk = m.y - t * kMaxTopK;
     uint4* dst = reinterpret_cast<uint4*>(a.dOut + (size_t)rowIdx * H);
-    if (src < 0 || src >= a.L.nranks || t < 0 || t >= a.T || kk >= a.k) {  // not a row of this pass: contributes nothing
+    if (r >= have || src < 0 || src >= a.L.nranks || t < 0 || t >= a.T || kk >= a.k) {  // not a row of this pass: contributes nothing
       for (int j = lane; j < H / 8; j += 32) dst[j] = make_uint4(0, 0, 0, 0);
       continue;
     }
     const float g = *reinterpret_cast<const float*>(a.gatePeer[src] + ((size_t)t * a.k + kk) * 4);
     const uint4* row = reinterpret_cast<const uint4*>(a.dyPeer[src] + (size_t)t * H * 2);
-    for (int j = lane; j < H / 8; j += 32) {
-      uint4 v = ldStream16(row + j);
-      __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+    for (int j = lane; j < H / 8; j += 128) {  // hidden is a multiple of 1024
+      uint4 v[4];
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const float2 f = __bfloat1622float2(h[i]);
-        h[i] = __floats2bfloat162_rn(g * f.x, g * f.y);
+      for (int u = 0; u < 4; u++) v[u] = ldStream16(row + j + 32 * u);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v[u]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float2 f = __bfloat1622float2(h[i]);
+          h[i] = __floats2bfloat162_rn(g * f.x, g * f.y);
+        }
+        dst[j + 32 * u] = v[u];
       }
-      dst[j] = v;
     }
   }
 }
 
-template <int BN, bool SWIGLU>
-__global__ void __launch_bounds__(gemm::kThreads, 1) groupedGemmKernel(const __grid_constant__ gemm::Params p, GroupPolicy<BN, SWIGLU> pol) {
-  extern __shared__ uint8_t smemRaw[];
-  __shared__ int prefix[kMaxLocalExperts + 1];
-  fillBlockPrefix(prefix, pol.cnt, pol.experts, pol.cap);
-  pol.prefix = prefix;
-  gemm::gemmCta<BN>(p, pol, blockIdx.x, gridDim.x, smemRaw);
+// SwiGLU backward over the rows that arrived, in place: gu [rows, 2 ffn] holds gate and up columns in turn per 128 and becomes its own
+// gradient given dAct [rows, ffn]. A warp per row. The rows up to the next multiple of 16, over which the weight-gradient GEMMs
+// reduce as well, become zeros in gu and in those GEMMs' other operands.
+struct SwigluGradArgs {
+  const uint32_t* cnt;
+  __nv_bfloat16* gu;
+  const __nv_bfloat16* dAct;
+  __nv_bfloat16* act;  // [rows, ffn]
+  __nv_bfloat16* xb;   // [rows, hidden]
+  int experts, cap, hidden, ffn;
+};
+__global__ void __launch_bounds__(256) epSwigluGrad(const SwigluGradArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  const int F = a.ffn;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (int e = 0, first = 0; e < a.experts; e++) {
+    const int have = min((int)a.cnt[e], a.cap), padded = (have + 15) & ~15;
+    // warps take the padded rows of all experts in turn
+    for (int r = (gw - first % nw + nw) % nw; r < padded; r += nw) {
+      const size_t row = (size_t)e * a.cap + r;
+      uint4* g4 = reinterpret_cast<uint4*>(a.gu + row * 2 * F);
+      if (r >= have) {
+        for (int j = lane; j < F / 4; j += 32) g4[j] = zero;
+        for (int j = lane; j < F / 8; j += 32) reinterpret_cast<uint4*>(a.act + row * F)[j] = zero;
+        for (int j = lane; j < a.hidden / 8; j += 32) reinterpret_cast<uint4*>(a.xb + row * a.hidden)[j] = zero;
+        continue;
+      }
+      const uint4* d4 = reinterpret_cast<const uint4*>(a.dAct + row * F);
+      for (int j = lane; j < F / 8; j += 32) {
+        const int at = (j >> 4) * 32 + (j & 15);  // 16 vectors of gate, then 16 of up
+        uint4 gv = g4[at], uv = g4[at + 16];
+        const uint4 dv = d4[j];
+        __nv_bfloat162 *g = reinterpret_cast<__nv_bfloat162*>(&gv), *u = reinterpret_cast<__nv_bfloat162*>(&uv);
+        const __nv_bfloat162* d = reinterpret_cast<const __nv_bfloat162*>(&dv);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float2 gf = __bfloat1622float2(g[i]), uf = __bfloat1622float2(u[i]), df = __bfloat1622float2(d[i]);
+          const float s0 = 1.f / (1.f + __expf(-gf.x)), s1 = 1.f / (1.f + __expf(-gf.y));
+          const float l0 = gf.x * s0, l1 = gf.y * s1;
+          g[i] = __floats2bfloat162_rn(df.x * uf.x * (s0 + l0 * (1.f - s0)), df.y * uf.y * (s1 + l1 * (1.f - s1)));
+          u[i] = __floats2bfloat162_rn(df.x * l0, df.y * l1);
+        }
+        g4[at] = gv;
+        g4[at + 16] = uv;
+      }
+    }
+    first += padded;
+  }
+}
+
+// Gradient with respect to the router logits [T, E]: the gate weights are the softmax over the k selected logits, so
+// w (dGate - sum dGate w) goes to the selected columns and zeros to all others. A warp per token.
+__global__ void __launch_bounds__(256) epRouterGrad(const float* __restrict__ topW, const int* __restrict__ topIdx, const float* __restrict__ dGate,
+                                                    float* __restrict__ dLogits, int T, int E, int k) {
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (t >= T) return;
+  float w[kMaxTopK], d[kMaxTopK], dot = 0.f;
+  int id[kMaxTopK];
+#pragma unroll
+  for (int r = 0; r < kMaxTopK; r++) {
+    w[r] = d[r] = 0.f;
+    id[r] = -1;
+    if (r < k) {
+      w[r] = topW[(size_t)t * k + r];
+      d[r] = dGate[(size_t)t * k + r];
+      id[r] = topIdx[(size_t)t * k + r];
+      dot += d[r] * w[r];
+    }
+  }
+  for (int c = lane; c < E; c += 32) {
+    float v = 0.f;
+#pragma unroll
+    for (int r = 0; r < kMaxTopK; r++)
+      if (id[r] == c) v = w[r] * (d[r] - dot);
+    dLogits[(size_t)t * E + c] = v;
+  }
 }
 
 }  // namespace ep
@@ -573,6 +514,7 @@ namespace {
 
 struct EpState {
   unsigned long long calls = 0;   // dispatches so far on this window
+  int rowsPerExpert = 0;          // of the latest one on average, were every rank to send as much as this one
   uint32_t* ticket = nullptr;     // device: CTA ticket + dropped-row counter
 };
 std::mutex gEpMu;
@@ -617,14 +559,33 @@ ncclResult_t checkShape(int expertsLocal, int cap, int hidden, int ffn, int k) {
   return ncclSuccess;
 }
 
-template <int BN, bool SW>
-cudaError_t launchGrouped(const gemm::Params& p, const GroupPolicy<BN, SW>& pol, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(groupedGemmKernel<BN, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm::Cfg<BN>::kSmemBytes);
-  if (e != cudaSuccess) return e;
-  int grid = gemm::smCount();
-  if (grid > p.tilesM * p.tilesN) grid = p.tilesM * p.tilesN;
-  groupedGemmKernel<BN, SW><<<grid, gemm::kThreads, gemm::Cfg<BN>::kSmemBytes, s>>>(p, pol);
-  return cudaGetLastError();
+// What the launches behind a dispatch need to know about it.
+struct Arrived {
+  EpLayout L;
+  int parity, rowsPerExpert;
+  const uint32_t* cnt;
+};
+ncclResult_t arrived(const char* what, Comm* c, const void* winSym, int expertsLocal, int cap, int hidden, int ffn, Arrived* a) {
+  a->L = makeLayout(c->nranks, expertsLocal, cap, hidden, ffn);
+  std::lock_guard<std::mutex> lk(gEpMu);
+  auto it = gEp.find(std::make_pair(c, winSym));
+  if (it == gEp.end() || it->second.calls == 0) BFAIL(ncclInvalidUsage, "%s: no dispatch has run on this window", what);
+  a->parity = (int)((it->second.calls - 1) & 1);
+  a->rowsPerExpert = it->second.rowsPerExpert;
+  a->cnt = (const uint32_t*)((const char*)winSym + a->L.cntOff) + (size_t)a->parity * expertsLocal;
+  return ncclSuccess;
+}
+
+// Up to 96 rows per expert on average the kernels with output features as MMA rows are faster, above CTA pairs. 32 experts, hidden 4096,
+// ffn 1024, whole forward pass: 16 rows 207 us against 262, 96 rows 254 against 271, 128 rows level, 256 rows 398 against 360;
+// with fp8 gate/up weights 157 against 240, 225 against 245, 270 against 253, 418 against 338; forward and backward 864
+// against 964, 1007 against 1013, 1062 against 1037, 1367 against 1248.
+bool fewRows(const Arrived& a) { return a.rowsPerExpert <= 96; }
+
+cudaError_t groupedRows(const Arrived& a, const void* x, const void* w, void* out, int N, int K, bool wMn, bool swiglu, cudaStream_t s) {
+  if (fewRows(a) && (!wMn || K % 64 == 0))
+    return gemmn::gemmNarrowGroupedBf16(x, w, out, a.cnt, a.L.expertsLocal, a.L.cap, a.rowsPerExpert, N, K, wMn, swiglu ? 256 : 0, s);
+  return gemm2::gemmPairGroupedRows(x, w, out, a.cnt, a.L.expertsLocal, a.L.cap, N, K, wMn, swiglu, s);
 }
 
 }  // namespace
@@ -639,7 +600,13 @@ ncclResult_t b200collEpRoute(const float* logits, int* topIdx, float* topW, int 
   if (!logits || !topIdx || !topW) BFAIL(ncclInvalidArgument, "b200collEpRoute: null buffer");
   if (E % 32 || E > 1024 || k < 1 || k > kMaxTopK || k > E) BFAIL(ncclInvalidArgument, "b200collEpRoute: E must be a multiple of 32 up to 1024, k in [1, 8]");
   if (T == 0) return ncclSuccess;
-  epRoute<<<(T + 7) / 8, 256, 0, stream>>>(logits, topIdx, topW, T, E, k);
+  const dim3 grid((T + 7) / 8);
+  if (E <= 32) epRoute<1><<<grid, 256, 0, stream>>>(logits, topIdx, topW, T, E, k);
+  else if (E <= 64) epRoute<2><<<grid, 256, 0, stream>>>(logits, topIdx, topW, T, E, k);
+  else if (E <= 128) epRoute<4><<<grid, 256, 0, stream>>>(logits, topIdx, topW, T, E, k);
+  else if (E <= 256) epRoute<8><<<grid, 256, 0, stream>>>(logits, topIdx, topW, T, E, k);
+  else if (E <= 512) epRoute<16><<<grid, 256, 0, stream>>>(logits, topIdx, topW, T, E, k);
+  else epRoute<32><<<grid, 256, 0, stream>>>(logits, topIdx, topW, T, E, k);
   BCUDA(cudaGetLastError());
   return ncclSuccess;
 }
@@ -665,6 +632,7 @@ ncclResult_t b200collEpDispatch(ncclComm_t comm, void* winSym, const void* xBf16
     }
     a.parity = (int)(st.calls & 1);
     a.doneValue = (uint32_t)(st.calls / 2 + 1);
+    st.rowsPerExpert = (int)std::min<long long>((long long)T * k / expertsLocal, cap);
     st.calls++;
     a.ticket = st.ticket;
     a.dropped = (int*)(st.ticket + 4);
@@ -677,8 +645,10 @@ ncclResult_t b200collEpDispatch(ncclComm_t comm, void* winSym, const void* xBf16
   DevComm dc = c->dev;
   dc.opSeq = ++c->opSeq;
   dc.stamp = nullptr;
-  int ctas = std::max(1, std::min((T + 7) / 8, 4 * gemm::smCount()));
-  epDispatch<<<ctas, 256, 0, stream>>>(a, dc);
+  // A warp per token, spread over the SMs before they share one (64 tokens on 8 SMs took 30 us); the kernel wants a thread per rank.
+  const int warps = std::max((c->nranks + 31) / 32, std::min(8, (T + gemm::smCount() - 1) / gemm::smCount()));
+  const int ctas = std::max(1, std::min((T + warps - 1) / warps, 4 * gemm::smCount()));
+  epDispatch<<<ctas, 32 * warps, 0, stream>>>(a, dc);
   BCUDA(cudaGetLastError());
   return ncclSuccess;
 }
@@ -694,67 +664,28 @@ static ncclResult_t epExperts(const char* what, ncclComm_t comm, void* winSym, c
   BCHECK(checkShape(expertsLocal, cap, hidden, ffn, 1));
   if (!winSym || !w13 || !w2 || (!fp8 && !xb) || !act) BFAIL(ncclInvalidArgument, "%s: null buffer", what);
   EpGuard g(c->cudaDev);
-  const EpLayout L = makeLayout(c->nranks, expertsLocal, cap, hidden, ffn);
-  int parity;
-  {
-    std::lock_guard<std::mutex> lk(gEpMu);
-    auto it = gEp.find(std::make_pair(c, (const void*)winSym));
-    if (it == gEp.end() || it->second.calls == 0) BFAIL(ncclInvalidUsage, "%s: no dispatch has run on this window", what);
-    parity = (int)((it->second.calls - 1) & 1);
-  }
-  const char* win = (const char*)winSym;
-  const uint32_t* cnt = (const uint32_t*)(win + L.cntOff) + (size_t)parity * expertsLocal;
-  const int rows = expertsLocal * cap;
-  const int wRows = 2 * ffn;
+  Arrived a;
+  BCHECK(arrived(what, c, winSym, expertsLocal, cap, hidden, ffn, &a));
+  char* win = (char*)winSym;
+  cudaError_t e;
   if (fp8) {
-    // GEMM 1: act = swiglu(dequant(rows) * dequant(w13)^T) on the window's payload.
-    gemm8::Params p{};
-    if (!gemm::makeTileMap(&p.mapA, win + L.payloadOff, rows, hidden, hidden, gemm::BM, 1) ||
-        !gemm::makeTileMap(&p.mapB, w13, (uint64_t)expertsLocal * wRows, hidden, hidden, gemm8::BN, 1))
-      BFAIL(ncclInvalidArgument, "%s: misaligned operands", what);
-    p.sA = (const float*)(win + L.scaleOff);
-    p.sB = w13Scales;
-    p.C = (__nv_bfloat16*)act;
-    p.M = rows; p.N = wRows; p.K = hidden; p.ldc = ffn;
-    p.tilesM = rows / gemm::BM; p.tilesN = wRows / gemm8::BN; p.kBlocks = hidden / 128;
-    p.err = gemm::errWord();
-    if (!p.err) BFAIL(ncclUnhandledCudaError, "%s: no error word", what);
-    GroupPolicy8 pol{cnt, expertsLocal, nullptr, cap, cap / gemm::BM, wRows, p.sA, hidden / 128, (__nv_bfloat16*)act, ffn, ffn};
-    cudaError_t e = cudaFuncSetAttribute(groupedGemmFp8Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm8::kSmemBytes);
-    if (e == cudaSuccess) {
-      int grid = gemm::smCount();
-      if (grid > p.tilesM * p.tilesN) grid = p.tilesM * p.tilesN;
-      groupedGemmFp8Kernel<<<grid, gemm8::kThreads, gemm8::kSmemBytes, stream>>>(p, pol);
-      e = cudaGetLastError();
-    }
-    if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "%s: first grouped GEMM failed to launch: %s", what, cudaGetErrorString(e));
+    // GEMM 1: act = swiglu(dequant(rows) * dequant(w13)^T) straight on the window's e4m3 rows and scales.
+    const char* rows8 = win + a.L.payloadOff;
+    const float* scales = (const float*)(win + a.L.scaleOff);
+    e = fewRows(a) ? gemmn8::gemmNarrowGroupedFp8(rows8, scales, w13, w13Scales, act, a.cnt, expertsLocal, cap, a.rowsPerExpert, 2 * ffn, hidden, true, stream)
+                      : gemm8p::gemmFp8PairGroupedSwiglu(rows8, scales, w13, w13Scales, act, a.cnt, expertsLocal, cap, 2 * ffn, hidden, stream);
   } else {
-    epDequant<<<4 * gemm::smCount(), 256, 0, stream>>>(win, L, parity, (__nv_bfloat16*)xb);
+    epDequant<<<8 * gemm::smCount(), 256, 0, stream>>>(win, a.L, a.parity, (__nv_bfloat16*)xb);
     BCUDA(cudaGetLastError());
-    // GEMM 1: act = swiglu(xb * w13^T), w13 [expertsLocal * 2 ffn, hidden] with gate/up interleaved per tile.
-    const int bn = wRows % 256 == 0 ? 256 : 128;
-    gemm::Params p{};
-    if (!gemm::makeTileMap(&p.mapA, xb, rows, hidden, hidden, gemm::BM, 2) || !gemm::makeTileMap(&p.mapB, w13, (uint64_t)expertsLocal * wRows, hidden, hidden, bn, 2))
-      BFAIL(ncclInvalidArgument, "%s: misaligned operands", what);
-    p.M = rows; p.N = wRows; p.K = hidden; p.tilesM = rows / gemm::BM; p.tilesN = wRows / bn; p.err = gemm::errWord();
-    cudaError_t e;
-    if (bn == 256) e = launchGrouped(p, GroupPolicy<256, true>{cnt, expertsLocal, nullptr, cap, cap / gemm::BM, wRows, (__nv_bfloat16*)act, ffn, ffn}, stream);
-    else e = launchGrouped(p, GroupPolicy<128, true>{cnt, expertsLocal, nullptr, cap, cap / gemm::BM, wRows, (__nv_bfloat16*)act, ffn, ffn}, stream);
-    if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "%s: first grouped GEMM failed to launch: %s", what, cudaGetErrorString(e));
+    // GEMM 1: act = swiglu(xb * w13^T), w13 [expertsLocal * 2 ffn, hidden] with gate and up rows in turn per 128.
+    e = groupedRows(a, xb, w13, act, 2 * ffn, hidden, false, true, stream);
   }
+  if (e == cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "%s: misaligned operands", what);
+  if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "%s: first grouped GEMM failed to launch: %s", what, cudaGetErrorString(e));
   // GEMM 2: out = act * w2^T, w2 [expertsLocal * hidden, ffn].
-  {
-    const int bn = hidden % 256 == 0 ? 256 : 128;
-    gemm::Params p{};
-    __nv_bfloat16* out = (__nv_bfloat16*)((char*)winSym + L.outOff);
-    if (!gemm::makeTileMap(&p.mapA, act, rows, ffn, ffn, gemm::BM, 2) || !gemm::makeTileMap(&p.mapB, w2, (uint64_t)expertsLocal * hidden, ffn, ffn, bn, 2))
-      BFAIL(ncclInvalidArgument, "%s: misaligned operands", what);
-    p.M = rows; p.N = hidden; p.K = ffn; p.tilesM = rows / gemm::BM; p.tilesN = hidden / bn; p.err = gemm::errWord();
-    cudaError_t e;
-    if (bn == 256) e = launchGrouped(p, GroupPolicy<256, false>{cnt, expertsLocal, nullptr, cap, cap / gemm::BM, hidden, out, hidden, hidden}, stream);
-    else e = launchGrouped(p, GroupPolicy<128, false>{cnt, expertsLocal, nullptr, cap, cap / gemm::BM, hidden, out, hidden, hidden}, stream);
-    if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "%s: second grouped GEMM failed to launch: %s", what, cudaGetErrorString(e));
-  }
+  e = groupedRows(a, act, w2, win + a.L.outOff, hidden, ffn, false, false, stream);
+  if (e == cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "%s: misaligned operands", what);
+  if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "%s: second grouped GEMM failed to launch: %s", what, cudaGetErrorString(e));
   return ncclSuccess;
 }
 
@@ -789,14 +720,6 @@ ncclResult_t b200collEpCombine(ncclComm_t comm, void* winSym, const int* topIdx,
 }
 
 // ---- backward pass ---------------------------------------------------------------------------------------------
-static ncclResult_t epLatestParity(const char* what, Comm* c, const void* winSym, int* parity) {
-  std::lock_guard<std::mutex> lk(gEpMu);
-  auto it = gEp.find(std::make_pair(c, winSym));
-  if (it == gEp.end() || it->second.calls == 0) BFAIL(ncclInvalidUsage, "%s: no dispatch has run on this window", what);
-  *parity = (int)((it->second.calls - 1) & 1);
-  return ncclSuccess;
-}
-
 // out[rows of expert e] = a[rows of expert e] * w[e]^T for every local expert, over the rows of the latest dispatch:
 // a [expertsLocal * cap, K], w [expertsLocal * wRows, K], out [expertsLocal * cap, wRows] (nullptr: the window's output
 // region, which needs wRows == hidden). Row blocks without tokens are skipped. The three GEMMs of the experts' backward
@@ -810,21 +733,48 @@ ncclResult_t b200collEpGroupedGemm(ncclComm_t comm, void* winSym, const void* a,
   if (wRows <= 0 || wRows % 128 || K <= 0 || K % 8) BFAIL(ncclInvalidArgument, "b200collEpGroupedGemm: weight rows %% 128 and K %% 8 must be 0");
   if (!out && wRows != hidden) BFAIL(ncclInvalidArgument, "b200collEpGroupedGemm: the window's output region holds rows of `hidden` columns");
   EpGuard g(c->cudaDev);
-  const EpLayout L = makeLayout(c->nranks, expertsLocal, cap, hidden, ffn);
-  int parity;
-  BCHECK(epLatestParity("b200collEpGroupedGemm", c, winSym, &parity));
-  const uint32_t* cnt = (const uint32_t*)((const char*)winSym + L.cntOff) + (size_t)parity * expertsLocal;
-  const int rows = expertsLocal * cap;
-  const int bn = wRows % 256 == 0 ? 256 : 128;
-  __nv_bfloat16* o = out ? (__nv_bfloat16*)out : (__nv_bfloat16*)((char*)winSym + L.outOff);
-  gemm::Params p{};
-  if (!gemm::makeTileMap(&p.mapA, a, rows, K, K, gemm::BM, 2) || !gemm::makeTileMap(&p.mapB, w, (uint64_t)expertsLocal * wRows, K, K, bn, 2))
-    BFAIL(ncclInvalidArgument, "b200collEpGroupedGemm: misaligned operands");
-  p.M = rows; p.N = wRows; p.K = K; p.tilesM = rows / gemm::BM; p.tilesN = wRows / bn; p.err = gemm::errWord();
-  cudaError_t e;
-  if (bn == 256) e = launchGrouped(p, GroupPolicy<256, false>{cnt, expertsLocal, nullptr, cap, cap / gemm::BM, wRows, o, wRows, wRows}, stream);
-  else e = launchGrouped(p, GroupPolicy<128, false>{cnt, expertsLocal, nullptr, cap, cap / gemm::BM, wRows, o, wRows, wRows}, stream);
+  Arrived r;
+  BCHECK(arrived("b200collEpGroupedGemm", c, winSym, expertsLocal, cap, hidden, ffn, &r));
+  const cudaError_t e = groupedRows(r, a, w, out ? out : (char*)winSym + r.L.outOff, wRows, K, false, false, stream);
+  if (e == cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "b200collEpGroupedGemm: misaligned operands");
   if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "b200collEpGroupedGemm: launch failed: %s", cudaGetErrorString(e));
+  return ncclSuccess;
+}
+
+// The experts' backward pass over the rows of the latest dispatch, given dOut (b200collEpGatherGrad) and what the forward pass left in xb
+// and act: the gradient of the rows goes to the window's output region, the weights' to dW13 and dW2 (every element is written).
+// gu [expertsLocal * cap, 2 ffn] and dAct [expertsLocal * cap, ffn] are scratch. No host round trip: the row counts stay on the device.
+ncclResult_t b200collEpExpertsBackward(ncclComm_t comm, void* winSym, const void* dOut, const void* w13, const void* w2, void* xb, void* act, void* gu, void* dAct,
+                                       void* dW13, void* dW2, int expertsLocal, int cap, int hidden, int ffn, cudaStream_t stream) {
+  Comm* c = asComm(comm);
+  BCHECK(commCheck(c));
+  BCHECK(checkShape(expertsLocal, cap, hidden, ffn, 1));
+  if (!winSym || !dOut || !w13 || !w2 || !xb || !act || !gu || !dAct || !dW13 || !dW2) BFAIL(ncclInvalidArgument, "b200collEpExpertsBackward: null buffer");
+  EpGuard g(c->cudaDev);
+  Arrived a;
+  BCHECK(arrived("b200collEpExpertsBackward", c, winSym, expertsLocal, cap, hidden, ffn, &a));
+  cudaError_t e = groupedRows(a, dOut, w2, dAct, ffn, hidden, true, false, stream);                          // dAct = dOut * w2
+  if (e == cudaSuccess) e = groupedRows(a, xb, w13, gu, 2 * ffn, hidden, false, false, stream);              // the pre-activations again
+  if (e == cudaSuccess) {
+    const SwigluGradArgs sg{a.cnt, (__nv_bfloat16*)gu, (const __nv_bfloat16*)dAct, (__nv_bfloat16*)act, (__nv_bfloat16*)xb, expertsLocal, cap, hidden, ffn};
+    epSwigluGrad<<<8 * gemm::smCount(), 256, 0, stream>>>(sg);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = groupedRows(a, gu, w13, (char*)winSym + a.L.outOff, hidden, 2 * ffn, true, false, stream);  // d rows = dGu * w13
+  if (e == cudaSuccess) e = gemm2::gemmPairGroupedSum(dOut, act, dW2, a.cnt, expertsLocal, cap, hidden, ffn, stream);
+  if (e == cudaSuccess) e = gemm2::gemmPairGroupedSum(gu, xb, dW13, a.cnt, expertsLocal, cap, 2 * ffn, hidden, stream);
+  if (e == cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "b200collEpExpertsBackward: misaligned operands");
+  if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "b200collEpExpertsBackward: launch failed: %s", cudaGetErrorString(e));
+  return ncclSuccess;
+}
+
+// d logits [T, E] from the gate weights, the expert ids and the gate weights' gradient, all [T, k].
+ncclResult_t b200collEpRouterGrad(const float* topW, const int* topIdx, const float* dGate, float* dLogits, int T, int E, int k, cudaStream_t stream) {
+  if (!topW || !topIdx || !dGate || !dLogits) BFAIL(ncclInvalidArgument, "b200collEpRouterGrad: null buffer");
+  if (k < 1 || k > kMaxTopK) BFAIL(ncclInvalidArgument, "b200collEpRouterGrad: top-k must be in [1, %d]", kMaxTopK);
+  if (T == 0) return ncclSuccess;
+  epRouterGrad<<<(T + 7) / 8, 256, 0, stream>>>(topW, topIdx, dGate, dLogits, T, E, k);
+  BCUDA(cudaGetLastError());
   return ncclSuccess;
 }
 
@@ -865,10 +815,12 @@ ncclResult_t b200collEpGatherGrad(ncclComm_t comm, void* winSym, const void* dyS
   if (!epPeers(c, dySym, (size_t)T * hidden * 2, dyPeer) || !epPeers(c, gateSym, (size_t)T * k * 4, gatePeer))
     BFAIL(ncclInvalidUsage, "b200collEpGatherGrad: dy and the gate weights must lie in symmetric memory");
   for (int r = 0; r < c->nranks; r++) { a.dyPeer[r] = dyPeer[r]; a.gatePeer[r] = gatePeer[r]; }
-  BCHECK(epLatestParity("b200collEpGatherGrad", c, winSym, &a.parity));
+  Arrived r;
+  BCHECK(arrived("b200collEpGatherGrad", c, winSym, expertsLocal, cap, hidden, ffn, &r));
+  a.parity = r.parity;
   a.win = (const char*)winSym; a.k = k; a.T = T; a.dOut = (__nv_bfloat16*)dOut;
   if (c->nranks > 1) BCHECK(b200collBarrier(comm, stream));
-  epGatherGrad<<<4 * gemm::smCount(), 256, 0, stream>>>(a);
+  epGatherGrad<<<8 * gemm::smCount(), 256, 0, stream>>>(a);
   BCUDA(cudaGetLastError());
   return ncclSuccess;
 }

@@ -89,5 +89,30 @@ cudaError_t gemmNarrowFp8(const void* X8, const float* sX, size_t sXBlock, size_
   return swiglu ? dispatch<true>(p, tn, tiles, 1, S, early, s) : dispatch<false>(p, tn, tiles, 1, S, early, s);
 }
 
+// C [groups * cap, N or N / 2] = X8 [groups * cap, K] * W8_g^T over the first cnt[g] rows of every group, `avg` of them as a rule;
+// sX [groups * cap][K / 128], N % 128 == 0, K at most kMaxBlocks blocks.
+cudaError_t gemmNarrowGroupedFp8(const void* X8, const float* sX, const void* W8, const float* sW, void* C, const uint32_t* cnt, int groups, int cap, int avg, int N,
+                                 int K, bool swiglu, cudaStream_t s) {
+  Params p{};
+  p.sX = sX;
+  p.sXBlock = 1;
+  p.sXRow = K / BK;
+  p.sW = sW;
+  p.C = (__nv_bfloat16*)C;
+  p.ldc = swiglu ? N / 2 : N;
+  p.M = cap;
+  p.N = N;
+  p.kBlocks = K / BK;
+  p.group.count = cnt;
+  p.group.cap = cap;
+  const int tn = 3 * avg <= 2 * 32 ? 32 : 64;
+  if (p.kBlocks > kMaxBlocks || !gemm::makeTileMap(&p.mapW, W8, (uint64_t)groups * N, K, K, BF, 1) || !gemm::makeTileMap(&p.mapX, X8, (uint64_t)groups * cap, K, K, tn, 1))
+    return cudaErrorInvalidValue;
+  p.err = gemm::errWord();
+  if (!p.err) return cudaErrorMemoryAllocation;
+  const int S = std::max(1, std::min({kMaxSplit, p.kBlocks, 256 / (N / BF * groups)}));
+  return swiglu ? dispatch<true>(p, tn, N / BF, groups, S, false, s) : dispatch<false>(p, tn, N / BF, groups, S, false, s);
+}
+
 }  // namespace gemmn8
 }  // namespace b200

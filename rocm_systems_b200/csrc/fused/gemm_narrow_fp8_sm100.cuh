@@ -148,9 +148,11 @@ __global__ void __launch_bounds__(kThreads, 2) gemmNarrowFp8Kernel(const __grid_
     {
       gridDependencyWait();
       const float* sW = p.sW + ((size_t)blockIdx.z * ((p.N + BF - 1) / BF) + tile) * p.kBlocks;
-      for (int i = et; i < (kb1 - kb0) * TN; i += 128) {
-        const int kb = kb0 + i / TN, t = i % TN;
-        scales[i] = t < tokens ? p.sX[(size_t)kb * p.sXBlock + (size_t)(xRow0 + t) * p.sXRow] * __ldg(sW + kb) : 0.f;
+      const int nb = kb1 - kb0;
+      const bool rowMajor = p.sXBlock == 1;  // neighbouring threads take what lies side by side in the table
+      for (int i = et; i < nb * TN; i += 128) {
+        const int t = rowMajor ? i / nb : i % TN, kb = rowMajor ? i % nb : i / TN;
+        scales[kb * TN + t] = t < tokens ? p.sX[(size_t)(kb0 + kb) * p.sXBlock + (size_t)(xRow0 + t) * p.sXRow] * __ldg(sW + kb0 + kb) : 0.f;
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
     }

@@ -70,7 +70,7 @@ int splitsFor(int tiles, int tokTiles, int kSteps) {
 namespace {
 
 cudaError_t run(Params& p, const void* X, const void* W, int xRows, int groups, int tn, int ldx, int ldw, bool wMn, cudaStream_t s) {
-  const bool okW = wMn ? gemm::makeTileMap(&p.mapW, W, p.K, p.N, ldw, 64, 2) : gemm::makeTileMap(&p.mapW, W, (uint64_t)groups * p.N, p.K, ldw, 64, 2);
+  const bool okW = wMn ? gemm::makeTileMap(&p.mapW, W, (uint64_t)groups * p.K, p.N, ldw, 64, 2) : gemm::makeTileMap(&p.mapW, W, (uint64_t)groups * p.N, p.K, ldw, 64, 2);
   if (!okW || !gemm::makeTileMap(&p.mapX, X, xRows, p.K, ldx, tn, 2)) return cudaErrorInvalidValue;
   p.err = gemm::errWord();
   if (!p.err) return cudaErrorMemoryAllocation;
@@ -93,6 +93,23 @@ cudaError_t gemmNarrowBf16(const void* X, const void* W, void* C, int M, int N, 
   p.K = K;
   p.gateUpTile = gateUpTile;
   return run(p, X, W, M, 1, M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128, ldx, ldw, wMn, s);
+}
+
+// C [groups * cap, N or N / 2] = X [groups * cap, K] * W_g^T over the first cnt[g] rows of every group, `avg` of them as a rule (it sizes the
+// token tile: most groups fit one, and W is read again for every further one). wMn: W_g is stored [K, N], K % 64 == 0.
+cudaError_t gemmNarrowGroupedBf16(const void* X, const void* W, void* C, const uint32_t* cnt, int groups, int cap, int avg, int N, int K, bool wMn, int gateUpTile,
+                                  cudaStream_t s) {
+  if (wMn && (gateUpTile || K % BK)) return cudaErrorInvalidValue;
+  Params p{};
+  p.C = (__nv_bfloat16*)C;
+  p.ldc = gateUpTile ? N / 2 : N;
+  p.M = cap;
+  p.N = N;
+  p.K = K;
+  p.gateUpTile = gateUpTile;
+  p.group.count = cnt;
+  p.group.cap = cap;
+  return run(p, X, W, groups * cap, groups, 3 * avg <= 2 * 32 ? 32 : 3 * avg <= 2 * 64 ? 64 : 128, K, wMn ? N : K, wMn, s);
 }
 
 }  // namespace gemmn

@@ -43,14 +43,14 @@ template <int TN> struct Cfg {
 };
 
 // Grouped form (the experts of a mixture): blockIdx.z is the group g, which owns rows [g * cap, g * cap + count[g]) of X and C and
-// rows [g * N, (g + 1) * N) of W. count == nullptr: one group of all M rows.
+// rows [g * N, (g + 1) * N) of W (stored [K, N]: rows [g * K, (g + 1) * K), K a multiple of 64). count == nullptr: one group of all M rows.
 struct Group {
   const uint32_t* count;
   int cap;
 };
 
 struct Params {
-  CUtensorMap mapW;  // K-major: [groups * N, K], box {64, 64}. MN-major: [K, N], box {64, 64}
+  CUtensorMap mapW;  // K-major: [groups * N, K], box {64, 64}. MN-major: [groups * K, N], box {64, 64}
   CUtensorMap mapX;  // [M, K], box {64, TN}
   __nv_bfloat16* C;
   int ldc;
@@ -145,8 +145,13 @@ __global__ void __launch_bounds__(kThreads, 2) gemmNarrowKernel(const __grid_con
     row0 = n0 / half * p.gateUpTile + n0 % half;
     row1 = row0 + half;
   }
-  row0 += (int)blockIdx.z * p.N;
-  row1 += (int)blockIdx.z * p.N;
+  int kOff = 0;  // reduction steps of W before those of this group
+  if constexpr (W_MN) {
+    kOff = (int)blockIdx.z * p.K;
+  } else {
+    row0 += (int)blockIdx.z * p.N;
+    row1 += (int)blockIdx.z * p.N;
+  }
   const int tok0 = blockIdx.y * TN;
   const int xRow0 = (int)blockIdx.z * p.group.cap;
   const int rows = p.group.count ? min((int)p.group.count[blockIdx.z], p.group.cap) : p.M;
@@ -185,7 +190,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemmNarrowKernel(const __grid_con
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           const int row = h == 0 ? row0 : row1;
-          if constexpr (W_MN) tmaLoad2d(sw + h * kHalfBytes, &p.mapW, row, k * BK, &full[stage]);
+          if constexpr (W_MN) tmaLoad2d(sw + h * kHalfBytes, &p.mapW, row, kOff + k * BK, &full[stage]);
           else tmaLoad2d(sw + h * kHalfBytes, &p.mapW, k * BK, row, &full[stage]);
         }
         tmaLoad2d(smemX + (size_t)stage * C::kXBytes, &p.mapX, k * BK, xRow0 + tok0, &full[stage]);

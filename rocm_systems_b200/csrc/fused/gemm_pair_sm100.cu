@@ -13,7 +13,7 @@ int pairsOnDevice() {
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return gemm::smCount() / 2;
   if (!pairs[dev]) {
-    auto kernel = gemmPairKernel<256, false, false>;
+    auto kernel = gemmPairKernel<256, false, false, false>;
     int n = 0;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<256>::kSmemBytes) == cudaSuccess) {
       cudaLaunchConfig_t q{};
@@ -37,9 +37,15 @@ int pairsOnDevice() {
 
 namespace {
 
-template <int BN, bool A_MN, bool B_MN>
-cudaError_t launchPair(const Params& p, int maxCtas, cudaStream_t s) {
-  auto kernel = gemmPairKernel<BN, A_MN, B_MN>;
+template <int BN, bool A_MN, bool B_MN, Mode MODE = kPlain, bool SWIGLU = false>
+auto pairKernel() {
+  if constexpr (MODE == kPlain) return &gemmPairKernel<BN, A_MN, B_MN, SWIGLU>;
+  else return &ep::groupedGemmKernel<A_MN, B_MN, MODE, SWIGLU>;
+}
+
+template <int BN, bool A_MN, bool B_MN, Mode MODE = kPlain, bool SWIGLU = false>
+cudaError_t launchPair(const Params& p, int tiles, int maxCtas, cudaStream_t s) {
+  auto kernel = pairKernel<BN, A_MN, B_MN, MODE, SWIGLU>();
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -51,7 +57,6 @@ cudaError_t launchPair(const Params& p, int maxCtas, cudaStream_t s) {
   }
   int pairs = pairsOnDevice();
   if (maxCtas > 0 && maxCtas / 2 < pairs) pairs = maxCtas / 2 > 0 ? maxCtas / 2 : 1;
-  const int tiles = p.tilesM * p.tilesN;
   if (tiles < pairs) pairs = tiles;
   kernel<<<2 * pairs, kThreads, Cfg<BN>::kSmemBytes, s>>>(p);  // cluster shape (2, 1, 1) is part of the kernel
   return cudaGetLastError();
@@ -59,8 +64,9 @@ cudaError_t launchPair(const Params& p, int maxCtas, cudaStream_t s) {
 
 template <int BN>
 cudaError_t dispatchMajor(const Params& p, bool aMn, bool bMn, int maxCtas, cudaStream_t s) {
-  if (aMn) return bMn ? launchPair<BN, true, true>(p, maxCtas, s) : launchPair<BN, true, false>(p, maxCtas, s);
-  return bMn ? launchPair<BN, false, true>(p, maxCtas, s) : launchPair<BN, false, false>(p, maxCtas, s);
+  const int tiles = p.tilesM * p.tilesN;
+  if (aMn) return bMn ? launchPair<BN, true, true>(p, tiles, maxCtas, s) : launchPair<BN, true, false>(p, tiles, maxCtas, s);
+  return bMn ? launchPair<BN, false, true>(p, tiles, maxCtas, s) : launchPair<BN, false, false>(p, tiles, maxCtas, s);
 }
 
 }  // namespace
@@ -89,6 +95,65 @@ cudaError_t gemmPairBf16(const void* A, const void* B, void* C, int M, int N, in
   p.err = gemm::errWord();
   if (!p.err) return cudaErrorMemoryAllocation;
   return bn == 256 ? dispatchMajor<256>(p, aMn, bMn, maxCtas, s) : dispatchMajor<128>(p, aMn, bMn, maxCtas, s);
+}
+
+// C [M, N / 2] = SwiGLU over A [M, K] * W [N, K]^T, all K-major and packed; W holds 128 gate and 128 up rows in turn, N % 256 == 0.
+cudaError_t gemmPairSwiglu(const void* A, const void* W, void* C, int M, int N, int K, cudaStream_t s) {
+  if (reinterpret_cast<uintptr_t>(C) & 15) return cudaErrorInvalidValue;
+  Params p{};
+  if (!gemm::makeTileMap(&p.mapA, A, M, K, K, BM, 2) || !gemm::makeTileMap(&p.mapB, W, N, K, K, 128, 2)) return cudaErrorInvalidValue;
+  p.C = (__nv_bfloat16*)C;
+  p.ldc = N / 2;
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.tilesM = (M + 2 * BM - 1) / (2 * BM);
+  p.tilesN = N / 256;
+  p.err = gemm::errWord();
+  if (!p.err) return cudaErrorMemoryAllocation;
+  return launchPair<256, false, false, kPlain, true>(p, p.tilesM * p.tilesN, 0, s);
+}
+
+// C [groups * cap, N or N / 2] = A [groups * cap, K] * W_g^T over the first cnt[g] rows of every group. wMn: W_g is stored [K, N] (K a
+// multiple of 128), else [N, K]. swiglu: gate and up rows in turn per 128, N % 256 == 0.
+cudaError_t gemmPairGroupedRows(const void* A, const void* W, void* C, const uint32_t* cnt, int groups, int cap, int N, int K, bool wMn, bool swiglu, cudaStream_t s) {
+  Params p{};
+  const bool okB = wMn ? gemm::makeTileMap(&p.mapB, W, (uint64_t)groups * K, N, N, 64, 2) : gemm::makeTileMap(&p.mapB, W, (uint64_t)groups * N, K, K, 128, 2);
+  if (!okB || !gemm::makeTileMap(&p.mapA, A, (uint64_t)groups * cap, K, K, BM, 2) || groups > kMaxGroups || (wMn && (swiglu || K % 128))) return cudaErrorInvalidValue;
+  p.C = (__nv_bfloat16*)C;
+  p.ldc = swiglu ? N / 2 : N;
+  p.N = N;
+  p.K = K;
+  p.tilesN = (N + 255) / 256;
+  p.cnt = cnt;
+  p.groups = groups;
+  p.cap = cap;
+  p.err = gemm::errWord();
+  if (!p.err) return cudaErrorMemoryAllocation;
+  const int tiles = groups * ((cap + 2 * BM - 1) / (2 * BM)) * p.tilesN;  // at most
+  if (swiglu) return launchPair<256, false, false, kRows, true>(p, tiles, 0, s);
+  return wMn ? launchPair<256, false, true, kRows>(p, tiles, 0, s) : launchPair<256, false, false, kRows>(p, tiles, 0, s);
+}
+
+// C [groups * M, N]: C_g = A[rows of g]^T * B[rows of g], A [groups * cap, M], B [groups * cap, N]; rows from cnt[g] to the next multiple
+// of 16 are zeros in both.
+cudaError_t gemmPairGroupedSum(const void* A, const void* B, void* C, const uint32_t* cnt, int groups, int cap, int M, int N, cudaStream_t s) {
+  Params p{};
+  if (!gemm::makeTileMap(&p.mapA, A, (uint64_t)groups * cap, M, M, 64, 2) || !gemm::makeTileMap(&p.mapB, B, (uint64_t)groups * cap, N, N, 64, 2))
+    return cudaErrorInvalidValue;
+  p.C = (__nv_bfloat16*)C;
+  p.ldc = N;
+  p.M = M;
+  p.N = N;
+  p.K = cap;
+  p.tilesM = (M + 2 * BM - 1) / (2 * BM);
+  p.tilesN = (N + 255) / 256;
+  p.cnt = cnt;
+  p.groups = groups;
+  p.cap = cap;
+  p.err = gemm::errWord();
+  if (!p.err) return cudaErrorMemoryAllocation;
+  return launchPair<256, true, true, kSum>(p, groups * p.tilesM * p.tilesN, 0, s);
 }
 
 }  // namespace gemm2

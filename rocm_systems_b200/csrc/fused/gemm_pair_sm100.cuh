@@ -16,6 +16,15 @@
 // arrive on the even CTA's `accEmpty`. Four epilogue warps per CTA drain tensor memory through a swizzled staging buffer
 // into 256-byte row segments while the next tile's main loop runs (two accumulators). Every wait is bounded; a CTA that
 // gives up still reaches the cluster barriers at the end.
+//
+// SWIGLU: B holds gate and up rows in turn per tile (BN / 2 gate rows, then the BN / 2 up rows of the same outputs) and the epilogue
+// writes silu(gate) * up, BN / 2 columns per tile.
+//
+// Two forms for the experts of a mixture, `cap` rows reserved per expert of which cnt[e] hold tokens (read on the device, so no
+// host round trip), each one launch whose persistent CTA pairs share the tiles of all experts:
+//   kRows  C[rows of e] = A[rows of e] * B_e^T over the 256-row blocks that hold tokens.
+//   kSum   C_e[M, N] = A[rows of e]^T * B[rows of e] (a weight gradient), reduced over the rows that hold tokens; the rows up to the
+//          next multiple of 16 must be zeros in both operands.
 #pragma once
 
 #include "gemm_sm100.cuh"
@@ -44,21 +53,65 @@ template <int BN> struct Cfg {
   static constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + 1024 + 256 + 4 * kEpiBytesPerWarp;
 };
 
+enum Mode { kPlain, kRows, kSum };
+constexpr int kMaxGroups = 64;
+
 struct Params {
-  CUtensorMap mapA;  // K-major: [M, K], box {64, 128}.   MN-major: [K, M], box {64, 64}
-  CUtensorMap mapB;  // K-major: [N, K], box {64, BN / 2}. MN-major: [K, N], box {64, 64}
+  CUtensorMap mapA;  // K-major: [M, K], box {64, 128}.   MN-major: [K, M], box {64, 64}.   kRows: [groups * cap, K]; kSum: [groups * cap, M]
+  CUtensorMap mapB;  // K-major: [N, K], box {64, BN / 2}. MN-major: [K, N], box {64, 64}.  kRows: groups of them in turn; kSum: [groups * cap, N]
   __nv_bfloat16* C;
   int ldc;
-  int M, N, K;
-  int tilesM, tilesN;  // tiles of 256 x BN
+  int M, N, K;         // kRows: N, K per group; kSum: M, N per group
+  int tilesM, tilesN;  // tiles of 256 x BN (kRows: tilesM unused; kSum: per group)
+  const uint32_t* cnt; // rows of every group (may exceed cap)
+  int groups, cap;
   int* err;
 };
 
-template <int BN, bool A_MN, bool B_MN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPairKernel(const __grid_constant__ Params p) {
+// One tile: first rows of the operands (for an operand stored MN-major its first column) and first reduction steps, 16-step
+// slices of the reduction, rows [cRow, cEnd) of C, column block.
+struct Tile {
+  int aRow, aK, bRow, bK, steps, cRow, cEnd, tn;
+};
+
+template <int BN, Mode MODE>
+__device__ __forceinline__ Tile tileAt(const Params& p, const int* prefix, int t) {
+  Tile o;
+  o.aK = o.bK = 0;
+  o.steps = (p.K + 15) / 16;
+  if constexpr (MODE == kPlain) {
+    int tm;
+    gemm::bandedCoord(t, p.tilesM, p.tilesN, tm, o.tn);
+    o.aRow = o.cRow = tm * 2 * BM;
+    o.cEnd = p.M;
+    o.bRow = o.tn * BN;
+  } else if constexpr (MODE == kRows) {
+    const int rb = t / p.tilesN;
+    o.tn = t - rb * p.tilesN;
+    int g = 0;
+    while (prefix[g + 1] <= rb) g++;
+    o.aRow = o.cRow = g * p.cap + (rb - prefix[g]) * 2 * BM;
+    o.cEnd = g * p.cap + min((int)p.cnt[g], p.cap);
+    o.bRow = o.tn * BN;
+    o.bK = g;  // the caller turns the group into rows of B
+  } else {
+    const int per = p.tilesM * p.tilesN, g = t / per;
+    int tm;
+    gemm::bandedCoord(t - g * per, p.tilesM, p.tilesN, tm, o.tn);
+    o.aRow = tm * 2 * BM;
+    o.bRow = o.tn * BN;
+    o.aK = o.bK = g * p.cap;
+    o.steps = (min((int)p.cnt[g], p.cap) + 15) / 16;
+    o.cRow = g * p.M + o.aRow;
+    o.cEnd = (g + 1) * p.M;
+  }
+  return o;
+}
+
+template <int BN, bool A_MN, bool B_MN, Mode MODE, bool SWIGLU>
+__device__ __forceinline__ void gemmPairCta(const Params& p, uint8_t* smemRaw) {
   using C = Cfg<BN>;
   using namespace sm100;
-  extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~(uintptr_t)1023);
   uint8_t* smemA = smem;
   uint8_t* smemB = smem + (size_t)kStages * C::kABytes;
@@ -69,6 +122,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPai
   uint64_t* accEmpty = accFull + 2;      // used in the even CTA only
   uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(accEmpty + 2);
   uint8_t* epiStage = reinterpret_cast<uint8_t*>(bars) + 256;
+
+  __shared__ int prefix[MODE == kRows ? kMaxGroups + 1 : 1];  // 256-row blocks with tokens before group g
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cr = clusterCtaRank();  // 0: issues the MMAs; 1: its partner
@@ -86,6 +141,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPai
       mbarInit(&accEmpty[b], 8);  // four epilogue warps in each CTA of the pair
     }
     fenceBarrierInit();
+    if constexpr (MODE == kRows) {
+      int acc = 0;
+      for (int g = 0; g < p.groups; g++) {
+        prefix[g] = acc;
+        acc += (min((int)p.cnt[g], p.cap) + 2 * BM - 1) / (2 * BM);
+      }
+      prefix[p.groups] = acc;
+    }
   }
   if (warp == 1) {
     tmemAllocPair(tmemSlot, C::kTmemCols);
@@ -98,8 +161,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPai
   tcFenceAfter();
   const uint32_t tmem = *tmemSlot;
 
-  const int numTiles = p.tilesM * p.tilesN;
-  const int kIters = (p.K + kSub * BK - 1) / (kSub * BK);
+  const int numTiles = MODE == kRows ? prefix[p.groups] * p.tilesN : MODE == kSum ? p.groups * p.tilesM * p.tilesN : p.tilesM * p.tilesN;
+  constexpr int kStageSteps = kSub * BK / 16;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
   if (warp == 0) {
@@ -108,10 +171,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPai
       uint32_t phase = 0;
       bool ok = true;
       for (int t = pair; t < numTiles && ok; t += npairs) {
-        int tm, tn;
-        gemm::bandedCoord(t, p.tilesM, p.tilesN, tm, tn);
-        const int aRow = tm * 2 * BM + (int)cr * BM;
-        const int bRow = tn * BN + (int)cr * (BN / 2);
+        const Tile o = tileAt<BN, MODE>(p, prefix, t);
+        const int aRow = o.aRow + (int)cr * BM;
+        const int bRow = o.bRow + (int)cr * (BN / 2) + (MODE == kRows && !B_MN ? o.bK * p.N : 0);
+        const int bK = MODE == kRows ? (B_MN ? o.bK * p.K : 0) : o.bK;
+        const int kIters = (o.steps + kStageSteps - 1) / kStageSteps;
         for (int k = 0; k < kIters; k++) {
           if (!mbarWait(&empty[stage], phase ^ 1, err, gemm::ERR_PRODUCER_EMPTY)) { ok = false; break; }
           const uint32_t fullAddr = mapToCta(smemAddr(&full[stage]), 0);
@@ -123,13 +187,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPai
             const int k0 = (k * kSub + h) * BK;  // a slice that starts beyond K reads zeros
             if constexpr (A_MN) {
 #pragma unroll
-              for (int c = 0; c < BM / 64; c++) tmaLoad2dPair(sa + h * C::kASub + c * kChunkBytes, &p.mapA, aRow + c * 64, k0, fullAddr);
+              for (int c = 0; c < BM / 64; c++) tmaLoad2dPair(sa + h * C::kASub + c * kChunkBytes, &p.mapA, aRow + c * 64, o.aK + k0, fullAddr);
             } else {
               tmaLoad2dPair(sa + h * C::kASub, &p.mapA, k0, aRow, fullAddr);
             }
             if constexpr (B_MN) {
 #pragma unroll
-              for (int c = 0; c < BN / 2 / 64; c++) tmaLoad2dPair(sb + h * C::kBSub + c * kChunkBytes, &p.mapB, bRow + c * 64, k0, fullAddr);
+              for (int c = 0; c < BN / 2 / 64; c++) tmaLoad2dPair(sb + h * C::kBSub + c * kChunkBytes, &p.mapB, bRow + c * 64, bK + k0, fullAddr);
             } else {
               tmaLoad2dPair(sb + h * C::kBSub, &p.mapB, k0, bRow, fullAddr);
             }
@@ -148,6 +212,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPai
       int it = 0;
       bool ok = true;
       for (int t = pair; t < numTiles && ok; t += npairs) {
+        const int steps = MODE == kSum ? tileAt<BN, MODE>(p, prefix, t).steps : (p.K + 15) / 16;
+        if (MODE == kSum && steps == 0) continue;  // a group without rows: the epilogue writes zeros by itself
+        const int kIters = (steps + kStageSteps - 1) / kStageSteps;
         const int b = it & 1;
         const uint32_t accPhase = (it >> 1) & 1;
         it++;
@@ -167,7 +234,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPai
               const uint32_t ah = aAddr + h * C::kASub, bh = bAddr + h * C::kBSub;
               const uint64_t da = A_MN ? smemDescSw128Mn(ah + kk * 2048, kChunkBytes) : smemDescSw128(ah + kk * 32);
               const uint64_t db = B_MN ? smemDescSw128Mn(bh + kk * 2048, kChunkBytes) : smemDescSw128(bh + kk * 32);
-              mmaF16Pair(d, da, db, idesc, (k | h | kk) != 0);
+              if (MODE != kSum || k * kStageSteps + h * (BK / 16) + kk < steps) mmaF16Pair(d, da, db, idesc, (k | h | kk) != 0);
             }
           }
           mmaCommitBoth(smemAddr(&empty[stage]));  // the stage is free in both CTAs once these MMAs have read it
@@ -181,22 +248,43 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPai
     int it = 0;
     bool ok = true;
     for (int t = pair; t < numTiles && ok; t += npairs) {
-      int tm, tn;
-      gemm::bandedCoord(t, p.tilesM, p.tilesN, tm, tn);
+      const Tile o = tileAt<BN, MODE>(p, prefix, t);
+      const int row0 = o.cRow + (int)cr * BM + q * 32;
+      uint8_t* sw = epiStage + (size_t)q * C::kEpiBytesPerWarp;
+      constexpr int kOut = SWIGLU ? BN / 2 : BN;  // output columns of a tile
+      const auto rowPtr = [&](int r) -> __nv_bfloat16* { return row0 + r < o.cEnd ? p.C + (size_t)(row0 + r) * p.ldc + (size_t)o.tn * kOut : nullptr; };
+      const int colLimit = (SWIGLU ? p.N / 2 : p.N) - o.tn * kOut;
+      if (MODE == kSum && o.steps == 0) {
+        for (int r = 0; r < 32; r++) {  // N is a multiple of 8
+          __nv_bfloat16* dst = rowPtr(r);
+          if (dst != nullptr && lane * 8 < min(colLimit, kOut)) reinterpret_cast<uint4*>(dst)[lane] = make_uint4(0, 0, 0, 0);
+        }
+        continue;
+      }
       const int b = it & 1;
       const uint32_t accPhase = (it >> 1) & 1;
       it++;
       if (!mbarWait(&accFull[b], accPhase, err, gemm::ERR_EPI_ACC_FULL)) { ok = false; break; }
       tcFenceAfter();
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN);
-      const int row0 = tm * 2 * BM + (int)cr * BM + q * 32;
       gemm::drainStaged(
-          epiStage + (size_t)q * C::kEpiBytesPerWarp, lane, BN, p.N - tn * BN,
+          sw, lane, kOut, colLimit,
           [&](int c, uint32_t(&acc)[32]) {
             tmemLoad32(taddr + c * 32, acc);
-            tmemLoadWait();
+            if constexpr (SWIGLU) {
+              uint32_t up[32];
+              tmemLoad32(taddr + BN / 2 + c * 32, up);
+              tmemLoadWait();
+#pragma unroll
+              for (int i = 0; i < 32; i++) {
+                const float g = __uint_as_float(acc[i]);
+                acc[i] = __float_as_uint(g / (1.f + __expf(-g)) * __uint_as_float(up[i]));
+              }
+            } else {
+              tmemLoadWait();
+            }
           },
-          [&](int r) -> __nv_bfloat16* { return row0 + r < p.M ? p.C + (size_t)(row0 + r) * p.ldc + (size_t)tn * BN : nullptr; });
+          rowPtr);
       tcFenceBefore();
       __syncwarp();
       if (lane == 0) mbarArriveCluster(mapToCta(smemAddr(&accEmpty[b]), 0));
@@ -209,5 +297,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPai
   if (warp == 1) tmemDeallocPair(tmem, C::kTmemCols);
 }
 
+template <int BN, bool A_MN, bool B_MN, bool SWIGLU>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmPairKernel(const __grid_constant__ Params p) {
+  extern __shared__ uint8_t smemRaw[];
+  gemmPairCta<BN, A_MN, B_MN, kPlain, SWIGLU>(p, smemRaw);
+}
+
 }  // namespace gemm2
+namespace ep {
+
+template <bool A_MN, bool B_MN, gemm2::Mode MODE, bool SWIGLU>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm2::kThreads, 1) groupedGemmKernel(const __grid_constant__ gemm2::Params p) {
+  extern __shared__ uint8_t smemRaw[];
+  gemm2::gemmPairCta<256, A_MN, B_MN, MODE, SWIGLU>(p, smemRaw);
+}
+
+}  // namespace ep
 }  // namespace b200

@@ -106,7 +106,7 @@ __device__ __forceinline__ void drainStaged(uint8_t* sw, int lane, int outCols, 
     const int chunksRow = colsHere / 8;       // 16-byte chunks per staged row (16 for a full group)
     const int sub = lane & 15, half = lane >> 4;
     const int validChunks = max(0, min(chunksRow, (colLimit - h * 128) / 8));
-#pragma unroll 1
+#pragma unroll 4
     for (int r2 = 0; r2 < 32; r2 += 2) {
       const int r = r2 + half;
       __nv_bfloat16* dst = rowPtr(r);

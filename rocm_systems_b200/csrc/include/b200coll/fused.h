@@ -65,7 +65,7 @@ ncclResult_t b200collEpRoute(const float* logits, int* topIdx, float* topW, int 
 ncclResult_t b200collEpDispatch(ncclComm_t comm, void* winSym, const void* xBf16, const int* topIdx, int* sentSlot, int T, int k,
                                 int expertsLocal, int cap, int hidden, int ffn, cudaStream_t stream);
 /* Dequantise the received rows and run the two grouped expert GEMMs (SwiGLU between them) on
- * tcgen05. w13 [expertsLocal * 2 ffn, hidden]: per expert, per 256 (128) rows, gate rows then up
+ * tcgen05. w13 [expertsLocal * 2 ffn, hidden]: per expert, per 256 rows, gate rows then up
  * rows; w2 [expertsLocal * hidden, ffn]. xb / act: scratch [expertsLocal * cap, hidden / ffn] bf16. */
 ncclResult_t b200collEpExperts(ncclComm_t comm, void* winSym, const void* w13, const void* w2, void* xb, void* act, int expertsLocal, int cap,
                                int hidden, int ffn, cudaStream_t stream);
@@ -89,7 +89,12 @@ ncclResult_t b200collEpCounts(ncclComm_t comm, void* winSym, int expertsLocal, i
  *                rank filled earlier on its stream; a barrier inside orders them before the pulls.
  *   GroupedGemm  out[rows of e] = a[rows of e] * w[e]^T per local expert (a [expertsLocal * cap, K], w [expertsLocal * wRows, K],
  *                out [expertsLocal * cap, wRows]; nullptr: the window's output region, wRows == hidden), skipping row blocks
- *                without tokens: with transposed weights, the experts' input-gradient GEMMs.
+ *                without tokens.
+ *   ExpertsBackward  the experts' whole backward pass given dOut and the xb / act that the forward pass left: the rows' gradient goes
+ *                to the window's output region, the weights' gradients to dW13 / dW2 (laid out like w13 / w2, every element is
+ *                written). gu [expertsLocal * cap, 2 ffn] and dAct [expertsLocal * cap, ffn] bf16 are scratch; xb and act rows past an
+ *                expert's count may be overwritten. The row counts are read on the device.
+ *   RouterGrad   d logits [T, E] fp32 from the gate weights, ids and dGate [T, k].
  * The input gradient is then b200collEpCombine with unit weights. */
 ncclResult_t b200collEpGateGrad(ncclComm_t comm, void* winSym, const void* dy, const int* topIdx, const int* sentSlot, float* dGate, int T, int k,
                                 int expertsLocal, int cap, int hidden, int ffn, cudaStream_t stream);
@@ -97,6 +102,9 @@ ncclResult_t b200collEpGatherGrad(ncclComm_t comm, void* winSym, const void* dyS
                                   int cap, int hidden, int ffn, cudaStream_t stream);
 ncclResult_t b200collEpGroupedGemm(ncclComm_t comm, void* winSym, const void* a, const void* w, void* out, int wRows, int K, int expertsLocal, int cap,
                                    int hidden, int ffn, cudaStream_t stream);
+ncclResult_t b200collEpExpertsBackward(ncclComm_t comm, void* winSym, const void* dOut, const void* w13, const void* w2, void* xb, void* act, void* gu,
+                                       void* dAct, void* dW13, void* dW2, int expertsLocal, int cap, int hidden, int ffn, cudaStream_t stream);
+ncclResult_t b200collEpRouterGrad(const float* topW, const int* topIdx, const float* dGate, float* dLogits, int T, int E, int k, cudaStream_t stream);
 
 /* ---- RMSNorm backward for callers that may not allocate device memory (no counterpart in the reference) -------------
  * dx [T, H] and dw [H] (both bf16) of y = x * rstd * w; the fp32 accumulator of dw is a fixed 32 KiB array inside the
