@@ -323,10 +323,13 @@ ncclResult_t b200collAgGemm(ncclComm_t comm, void* xSym, const void* w, void* ou
   DevGuard2 g(c->cudaDev);
   // One rank gathers nothing: the plain GEMMs take the call where they have its epilogue. Without SwiGLU that is the CTA-pair
   // kernel (4096 x 4096 x 6144: 0.14 ms against 0.16 for the one-CTA kernel below); with it the few-row kernel, whose rule
-  // says where (128 x 28672 x 4096: 47 us against 49.5, and half the device stays idle on smaller weights).
-  if (n == 1 && (!swiglu || gemmn::prefersNarrow(M, wRows))) {
-    const cudaError_t e = swiglu ? gemmn::gemmNarrowBf16(xSym, w, out, M, wRows, K, K, K, wRows / 2, false, bn, stream)
-                                 : gemm2::gemmPairBf16(xSym, w, out, M, wRows, K, K, K, wRows, false, false, 0, 0, stream);
+  // says where (128 x 28672 x 4096: 47 us against 49.5, and half the device stays idle on smaller weights), else CTA pairs if
+  // gate and up rows take turns per 128.
+  if (n == 1 && (!swiglu || bn == 256 || gemmn::prefersNarrow(M, wRows))) {
+    cudaError_t e;
+    if (!swiglu) e = gemm2::gemmPairBf16(xSym, w, out, M, wRows, K, K, K, wRows, false, false, 0, 0, stream);
+    else if (gemmn::prefersNarrow(M, wRows)) e = gemmn::gemmNarrowBf16(xSym, w, out, M, wRows, K, K, K, wRows / 2, false, bn, stream);
+    else e = gemm2::gemmPairSwiglu(xSym, w, out, M, wRows, K, stream);
     if (e == cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "b200collAgGemm: operands must be 16-byte aligned with rows a multiple of 16 bytes");
     if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "b200collAgGemm launch failed: %s", cudaGetErrorString(e));
     return ncclSuccess;

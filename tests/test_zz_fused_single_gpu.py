@@ -46,3 +46,10 @@ def test_expert_parallel_layer_with_fp8_experts_on_one_rank():
 def test_device_initiated_layer_on_one_pe():
     """put+signal to itself, the atomics on its own words, the barrier of one: the device API's code paths on one GPU."""
     _launch(1, 29884, "shmem_worker.py", timeout=600)
+
+
+def test_tensor_parallel_mlp_on_one_rank_at_the_plain_gemms_sizes():
+    """Sizes that the plain CTA-pair GEMMs with the SwiGLU epilogue take on one rank (more than a round of 256 x 256 tiles, an odd number of
+    128-row blocks, a reduction that is no multiple of 256)."""
+    _launch(1, 29890, "tp_worker.py", "--rows", "640", "--hidden", "1152", "--ffn", "4224", timeout=600)
+    _launch(1, 29891, "tp_worker.py", "--fp8", "--rows", "1152", "--hidden", "1152", "--ffn", "4224", timeout=600)
