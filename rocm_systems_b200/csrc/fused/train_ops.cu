@@ -367,8 +367,13 @@ __global__ void __launch_bounds__(kThreads) swigluBwd(const __nv_bfloat16* __res
 // One CTA per token row: pass 1 finds max and sum(exp) online, then the row is rewritten in place
 // with (softmax - onehot) * gradScale. loss[row] = logsumexp - logit[target]. Rows whose target is
 // negative are ignored (zero gradient, zero loss).
-__global__ void __launch_bounds__(1024) crossEntropyFwdBwd(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
-                                                           float* __restrict__ lossPerRow, int V, size_t rowStride, float gradScale) {
+//
+// Four 16-byte loads of a thread are in flight at a time, in both passes: with one, 2048 threads kept 32 KB of an SM's loads under
+// way, a third of what the memory's latency asks for (4096 x 128256: 609 us, now 533 - 574).
+constexpr int kXentThreads = 512;
+constexpr int kXentUnroll = 4;
+__global__ void __launch_bounds__(kXentThreads, 2) crossEntropyFwdBwd(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
+                                                                   float* __restrict__ lossPerRow, int V, size_t rowStride, float gradScale) {
   __shared__ float sh[32];
   const size_t row = blockIdx.x;
   __nv_bfloat16* lr = logits + row * rowStride;
@@ -376,53 +381,71 @@ __global__ void __launch_bounds__(1024) crossEntropyFwdBwd(__nv_bfloat16* __rest
   const int nvec = V >> 3;
   Bf8* lv = reinterpret_cast<Bf8*>(lr);
   float m = -INFINITY, s = 0.f;
-  for (int j = threadIdx.x; j < nvec; j += blockDim.x) {
-    float f[8];
-    unpack8(lv[j], f);
-    float lm = f[0];
+  for (int j0 = threadIdx.x; j0 < nvec; j0 += kXentUnroll * kXentThreads) {
+    Bf8 raw[kXentUnroll];
 #pragma unroll
-    for (int k = 1; k < 8; k++) lm = fmaxf(lm, f[k]);
-    const float nm = fmaxf(m, lm);
-    float acc = 0.f;
+    for (int u = 0; u < kXentUnroll; u++)
+      if (j0 + u * kXentThreads < nvec) raw[u] = lv[j0 + u * kXentThreads];
 #pragma unroll
-    for (int k = 0; k < 8; k++) acc += __expf(f[k] - nm);
-    s = s * __expf(m - nm) + acc;
-    m = nm;
+    for (int u = 0; u < kXentUnroll; u++) {
+      if (j0 + u * kXentThreads >= nvec) break;
+      float f[8];
+      unpack8(raw[u], f);
+      float lm = f[0];
+#pragma unroll
+      for (int k = 1; k < 8; k++) lm = fmaxf(lm, f[k]);
+      const float nm = fmaxf(m, lm);
+      float acc = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; k++) acc += __expf(f[k] - nm);
+      s = s * __expf(m - nm) + acc;
+      m = nm;
+    }
   }
-  for (int j = (nvec << 3) + threadIdx.x; j < V; j += blockDim.x) {  // ragged tail
+  for (int j = (nvec << 3) + threadIdx.x; j < V; j += kXentThreads) {  // ragged tail
     const float f = __bfloat162float(lr[j]);
     const float nm = fmaxf(m, f);
     s = s * __expf(m - nm) + __expf(f - nm);
     m = nm;
   }
-  const float gm = blockMax<1024>(m, sh);
+  const float gm = blockMax<kXentThreads>(m, sh);
   s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
-  const float gs = blockSum<1024>(s, sh);
+  const float gs = blockSum<kXentThreads>(s, sh);
   const float lse = gm + __logf(gs);
   if (tgt < 0 || tgt >= V) {
     if (threadIdx.x == 0) lossPerRow[row] = 0.f;
-    for (int j = threadIdx.x; j < nvec; j += blockDim.x) {
+    for (int j = threadIdx.x; j < nvec; j += kXentThreads) {
       float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       lv[j] = pack8(z);
     }
-    for (int j = (nvec << 3) + threadIdx.x; j < V; j += blockDim.x) lr[j] = __float2bfloat16(0.f);
+    for (int j = (nvec << 3) + threadIdx.x; j < V; j += kXentThreads) lr[j] = __float2bfloat16(0.f);
     return;
   }
   if (threadIdx.x == 0) lossPerRow[row] = lse - __bfloat162float(lr[tgt]);
   __syncthreads();  // the target logit is read before anyone overwrites it
   const float inv = 1.f / gs;
-  for (int j = threadIdx.x; j < nvec; j += blockDim.x) {
-    float f[8];
-    unpack8(lv[j], f);
+  const int tvec = (int)(tgt >> 3), tlane = (int)(tgt & 7);
+  for (int j0 = threadIdx.x; j0 < nvec; j0 += kXentUnroll * kXentThreads) {
+    Bf8 raw[kXentUnroll];
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      float p = __expf(f[k] - gm) * inv;
-      if ((long long)(j * 8 + k) == tgt) p -= 1.f;
-      f[k] = p * gradScale;
+    for (int u = 0; u < kXentUnroll; u++)
+      if (j0 + u * kXentThreads < nvec) raw[u] = lv[j0 + u * kXentThreads];
+#pragma unroll
+    for (int u = 0; u < kXentUnroll; u++) {
+      const int j = j0 + u * kXentThreads;
+      if (j >= nvec) break;
+      float f[8];
+      unpack8(raw[u], f);
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        float p = __expf(f[k] - gm) * inv;
+        if (j == tvec && k == tlane) p -= 1.f;
+        f[k] = p * gradScale;
+      }
+      lv[j] = pack8(f);
     }
-    lv[j] = pack8(f);
   }
-  for (int j = (nvec << 3) + threadIdx.x; j < V; j += blockDim.x) {
+  for (int j = (nvec << 3) + threadIdx.x; j < V; j += kXentThreads) {
     float p = __expf(__bfloat162float(lr[j]) - gm) * inv;
     if ((long long)j == tgt) p -= 1.f;
     lr[j] = __float2bfloat16(p * gradScale);
@@ -443,43 +466,76 @@ __device__ __forceinline__ float4 loadGrad4(const __nv_bfloat16* g, size_t i) {
 __device__ __forceinline__ float loadGrad1(const float* g, size_t i) { return g[i]; }
 __device__ __forceinline__ float loadGrad1(const __nv_bfloat16* g, size_t i) { return __bfloat162float(g[i]); }
 
-template <typename G>
-__global__ void __launch_bounds__(kThreads) adamwKernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
-                                                        const G* __restrict__ grad, __nv_bfloat16* __restrict__ param, size_t n, float lr,
-                                                        float b1, float b2, float eps, float wd, float bc1, float bc2, float gradScale) {
-  const size_t nvec = n >> 2;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (size_t)gridDim.x * blockDim.x) {
-    float4 w4 = reinterpret_cast<float4*>(master)[i];
-    float4 m4 = reinterpret_cast<float4*>(m)[i];
-    float4 v4 = reinterpret_cast<float4*>(v)[i];
-    float4 g4 = loadGrad4(grad, i);
-    float* w = &w4.x; float* mm = &m4.x; float* vv = &v4.x; float* g = &g4.x;
+struct AdamHyper {
+  float lr, b1, b2, eps, wd, bc1, bc2, gradScale;
+};
+__device__ __forceinline__ void adamwUpdate4(float* master, float* m, float* v, __nv_bfloat16* param, size_t i, const float4& g4, const AdamHyper& h) {
+  float4 w4 = reinterpret_cast<float4*>(master)[i];
+  float4 m4 = reinterpret_cast<float4*>(m)[i];
+  float4 v4 = reinterpret_cast<float4*>(v)[i];
+  float* w = &w4.x; float* mm = &m4.x; float* vv = &v4.x; const float* g = &g4.x;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const float gk = g[k] * gradScale;
-      mm[k] = b1 * mm[k] + (1.f - b1) * gk;
-      vv[k] = b2 * vv[k] + (1.f - b2) * gk * gk;
-      const float upd = (mm[k] / bc1) / (sqrtf(vv[k] / bc2) + eps);
-      w[k] = w[k] - lr * (upd + wd * w[k]);
-    }
-    reinterpret_cast<float4*>(master)[i] = w4;
-    reinterpret_cast<float4*>(m)[i] = m4;
-    reinterpret_cast<float4*>(v)[i] = v4;
-    __nv_bfloat162 p0 = __floats2bfloat162_rn(w4.x, w4.y), p1 = __floats2bfloat162_rn(w4.z, w4.w);
-    uint2 packed;
-    packed.x = *reinterpret_cast<uint32_t*>(&p0);
-    packed.y = *reinterpret_cast<uint32_t*>(&p1);
-    reinterpret_cast<uint2*>(param)[i] = packed;
+  for (int k = 0; k < 4; k++) {
+    const float gk = g[k] * h.gradScale;
+    mm[k] = h.b1 * mm[k] + (1.f - h.b1) * gk;
+    vv[k] = h.b2 * vv[k] + (1.f - h.b2) * gk * gk;
+    // Moments that are zero still, as those of table rows without a token so far, move nothing; dividing them takes the slow
+    // path of division and square root (525 M such elements: 3.9 ms, 2.4 without).
+    float upd = 0.f;
+    if (mm[k] != 0.f || vv[k] != 0.f || !(h.eps > 0.f)) upd = (mm[k] / h.bc1) / (sqrtf(vv[k] / h.bc2) + h.eps);
+    w[k] = w[k] - h.lr * (upd + h.wd * w[k]);
   }
+  reinterpret_cast<float4*>(master)[i] = w4;
+  reinterpret_cast<float4*>(m)[i] = m4;
+  reinterpret_cast<float4*>(v)[i] = v4;
+  __nv_bfloat162 p0 = __floats2bfloat162_rn(w4.x, w4.y), p1 = __floats2bfloat162_rn(w4.z, w4.w);
+  uint2 packed;
+  packed.x = *reinterpret_cast<uint32_t*>(&p0);
+  packed.y = *reinterpret_cast<uint32_t*>(&p1);
+  reinterpret_cast<uint2*>(param)[i] = packed;
+}
+
+template <typename G>
+__global__ void __launch_bounds__(kThreads) adamwKernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v, const G* __restrict__ grad,
+                                        __nv_bfloat16* __restrict__ param, size_t n, const AdamHyper h) {
+  const size_t nvec = n >> 2;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (size_t)gridDim.x * blockDim.x)
+    adamwUpdate4(master, m, v, param, i, loadGrad4(grad, i), h);
   for (size_t i = (nvec << 2) + (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float gk = loadGrad1(grad, i) * gradScale;
-    const float mk = b1 * m[i] + (1.f - b1) * gk;
-    const float vk = b2 * v[i] + (1.f - b2) * gk * gk;
-    const float wk = master[i] - lr * ((mk / bc1) / (sqrtf(vk / bc2) + eps) + wd * master[i]);
+    const float gk = loadGrad1(grad, i) * h.gradScale;
+    const float mk = h.b1 * m[i] + (1.f - h.b1) * gk;
+    const float vk = h.b2 * v[i] + (1.f - h.b2) * gk * gk;
+    const float wk = master[i] - h.lr * ((mk / h.bc1) / (sqrtf(vk / h.bc2) + h.eps) + h.wd * master[i]);
     m[i] = mk;
     v[i] = vk;
     master[i] = wk;
     param[i] = __float2bfloat16(wk);
+  }
+}
+
+// The update of an embedding table [vocab, H], split by whether the batch has a token of that row: owner[id] is the first such token,
+// kNoToken without one. Rows without a token have gradient zero, so they need no gradient buffer (zero-filling and reading one took 8 of
+// the 34 bytes per element) and can be updated before the backward pass has come down to the embedding. TOUCHED: the
+// rows of the T tokens that own one, gradient in row t of grad [T, H].
+constexpr int kNoToken = 0x7f7f7f7f;
+template <bool TOUCHED>
+__global__ void __launch_bounds__(kThreads) adamwRowsKernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ grad,
+                                            __nv_bfloat16* __restrict__ param, const int* __restrict__ owner, const long long* __restrict__ tokens,
+                                            long long rows, int hv, const AdamHyper h) {
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  const long long rStep = (long long)(stride / hv);
+  const int jStep = (int)(stride % hv);
+  long long r = (long long)(first / hv);
+  for (int j = (int)(first % hv); r < rows;) {
+    const long long id = TOUCHED ? tokens[r] : r;
+    if (owner[id] == (TOUCHED ? (int)r : kNoToken))
+      adamwUpdate4(master, m, v, param, (size_t)id * hv + j, TOUCHED ? reinterpret_cast<const float4*>(grad)[(size_t)r * hv + j] : make_float4(0.f, 0.f, 0.f, 0.f), h);
+    r += rStep;
+    j += jStep;
+    if (j >= hv) {
+      j -= hv;
+      r++;
+    }
   }
 }
 
@@ -492,11 +548,15 @@ __global__ void __launch_bounds__(kThreads) embeddingFwd(const long long* __rest
   Bf8* dst = reinterpret_cast<Bf8*>(out + t * H);
   for (int j = threadIdx.x; j < (H >> 3); j += blockDim.x) dst[j] = src[j];
 }
-// dtable[tok] += dout[t] (fp32 table gradient; rows repeat, so atomics)
+__global__ void __launch_bounds__(kThreads) embeddingOwner(const long long* __restrict__ tokens, int* __restrict__ owner, int T) {
+  const int t = blockIdx.x * kThreads + threadIdx.x;
+  if (t < T) atomicMin(owner + tokens[t], t);
+}
+// dtable[tok] += dout[t] (fp32 table gradient; rows repeat, so atomics). owner != nullptr: into row owner[tok] of a [T, H] buffer.
 __global__ void __launch_bounds__(kThreads) embeddingBwd(const long long* __restrict__ tokens, const __nv_bfloat16* __restrict__ dout,
-                                                         float* __restrict__ dtable, int H) {
+                                                         float* __restrict__ dtable, const int* __restrict__ owner, int H) {
   const size_t t = blockIdx.x;
-  const long long tok = tokens[t];
+  const long long tok = owner ? owner[tokens[t]] : tokens[t];
   const __nv_bfloat162* src = reinterpret_cast<const __nv_bfloat162*>(dout + t * H);
   float* dst = dtable + (size_t)tok * H;
   for (int j = threadIdx.x; j < (H >> 1); j += blockDim.x) {
@@ -633,15 +693,18 @@ int b200ops_swiglu_bwd(const void* gu, const void* dout, void* dgu, long long T,
 int b200ops_cross_entropy(void* logits, const long long* targets, float* lossPerRow, long long T, int V, long long rowStride, float gradScale, cudaStream_t s) {
   if (rowStride % 8) return (int)cudaErrorInvalidValue;
   if (T == 0) return 0;
-  crossEntropyFwdBwd<<<(unsigned)T, 1024, 0, s>>>((__nv_bfloat16*)logits, targets, lossPerRow, V, (size_t)rowStride, gradScale);
+  crossEntropyFwdBwd<<<(unsigned)T, kXentThreads, 0, s>>>((__nv_bfloat16*)logits, targets, lossPerRow, V, (size_t)rowStride, gradScale);
   return (int)cudaGetLastError();
+}
+
+static AdamHyper adamHyper(float lr, float b1, float b2, float eps, float wd, int step, float gradScale) {
+  return {lr, b1, b2, eps, wd, 1.f - powf(b1, (float)step), 1.f - powf(b2, (float)step), gradScale};
 }
 
 int b200ops_adamw(float* master, float* m, float* v, const float* grad, void* param, long long n, float lr, float b1, float b2, float eps, float wd,
                   int step, float gradScale, cudaStream_t s) {
   if (n == 0) return 0;
-  const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
-  adamwKernel<float><<<gridFor((size_t)n, 4), kThreads, 0, s>>>(master, m, v, grad, (__nv_bfloat16*)param, (size_t)n, lr, b1, b2, eps, wd, bc1, bc2, gradScale);
+  adamwKernel<float><<<gridFor((size_t)n, 4), kThreads, 0, s>>>(master, m, v, grad, (__nv_bfloat16*)param, (size_t)n, adamHyper(lr, b1, b2, eps, wd, step, gradScale));
   return (int)cudaGetLastError();
 }
 
@@ -650,9 +713,35 @@ int b200ops_adamw_bf16g(float* master, float* m, float* v, const void* grad, voi
                         float wd, int step, float gradScale, cudaStream_t s) {
   if (n == 0) return 0;
   if ((uintptr_t)grad & 7) return (int)cudaErrorInvalidValue;
-  const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
-  adamwKernel<__nv_bfloat16><<<gridFor((size_t)n, 4), kThreads, 0, s>>>(master, m, v, (const __nv_bfloat16*)grad, (__nv_bfloat16*)param, (size_t)n, lr, b1, b2,
-                                                                         eps, wd, bc1, bc2, gradScale);
+  adamwKernel<__nv_bfloat16><<<gridFor((size_t)n, 4), kThreads, 0, s>>>(master, m, v, (const __nv_bfloat16*)grad, (__nv_bfloat16*)param, (size_t)n,
+                                                                          adamHyper(lr, b1, b2, eps, wd, step, gradScale));
+  return (int)cudaGetLastError();
+}
+
+// owner[id] (int32 [vocab]) = the first of the T tokens with that id, 0x7f7f7f7f without one.
+int b200ops_embedding_owner(const long long* tokens, int* owner, long long T, long long vocab, cudaStream_t s) {
+  if (T >= kNoToken) return (int)cudaErrorInvalidValue;
+  const cudaError_t e = cudaMemsetAsync(owner, 0x7f, (size_t)vocab * 4, s);
+  if (e != cudaSuccess || T == 0) return (int)e;
+  embeddingOwner<<<(unsigned)((T + kThreads - 1) / kThreads), kThreads, 0, s>>>(tokens, owner, (int)T);
+  return (int)cudaGetLastError();
+}
+// dRows [T, H] (fp32, zeroed by the caller): the table gradient of token t's row is summed into row owner[tokens[t]].
+int b200ops_embedding_bwd_owned(const long long* tokens, const void* dout, float* dRows, const int* owner, long long T, int H, cudaStream_t s) {
+  if (H % 2) return (int)cudaErrorInvalidValue;
+  if (T == 0) return 0;
+  embeddingBwd<<<(unsigned)T, kThreads, 0, s>>>(tokens, (const __nv_bfloat16*)dout, dRows, owner, H);
+  return (int)cudaGetLastError();
+}
+// AdamW on the rows of a table [vocab, H] that have no token (tokens == nullptr, gradient zero) or that one of the T tokens owns (grad [T, H]).
+int b200ops_adamw_rows(float* master, float* m, float* v, const float* grad, void* param, const int* owner, const long long* tokens, long long rows, int H, float lr,
+                       float b1, float b2, float eps, float wd, int step, cudaStream_t s) {
+  if (H % 4) return (int)cudaErrorInvalidValue;
+  if (rows == 0) return 0;
+  const AdamHyper h = adamHyper(lr, b1, b2, eps, wd, step, 1.f);
+  const int grid = gridFor((size_t)rows * H, 4);
+  if (tokens) adamwRowsKernel<true><<<grid, kThreads, 0, s>>>(master, m, v, grad, (__nv_bfloat16*)param, owner, tokens, rows, H / 4, h);
+  else adamwRowsKernel<false><<<grid, kThreads, 0, s>>>(master, m, v, nullptr, (__nv_bfloat16*)param, owner, nullptr, rows, H / 4, h);
   return (int)cudaGetLastError();
 }
 
@@ -665,7 +754,7 @@ int b200ops_embedding_fwd(const long long* tokens, const void* table, void* out,
 int b200ops_embedding_bwd(const long long* tokens, const void* dout, float* dtable, long long T, int H, cudaStream_t s) {
   if (H % 2) return (int)cudaErrorInvalidValue;
   if (T == 0) return 0;
-  embeddingBwd<<<(unsigned)T, kThreads, 0, s>>>(tokens, (const __nv_bfloat16*)dout, dtable, H);
+  embeddingBwd<<<(unsigned)T, kThreads, 0, s>>>(tokens, (const __nv_bfloat16*)dout, dtable, nullptr, H);
   return (int)cudaGetLastError();
 }
 

@@ -274,6 +274,9 @@ class LlamaTrainer:
             logits = mm_nt(hn.detach(), w_out)
             loss_rows = ops.cross_entropy_inplace(logits, tgt, 1.0 / T)
             loss = loss_rows.mean()
+            if eng.updates_rows:  # what no token of this batch touches of the embedding is updated beside the backward pass
+                owner = ops.embedding_owner(tok, cfg.vocab)
+                eng.update_idle_rows(self.embed, owner, cfg.hidden)
             eng.alloc_grad(self.head)
             dhn = mm_nt(logits, w_out.t())
             mm_nt(logits.t(), hn.detach().t(), out=self.head.grad_view("out"))
@@ -314,9 +317,14 @@ class LlamaTrainer:
                     eng.release(u)
 
             # ---- embedding gradient (fp32, rows repeat) ----
-            dtable = torch.zeros(self.embed.padded, dtype=torch.float32, device=self.device)
-            ops.embedding_bwd_(tok, g, dtable[: cfg.vocab * cfg.hidden].view(cfg.vocab, cfg.hidden))
-            eng.reduce_and_step(self.embed, fp32_full_grad=dtable)
+            if eng.updates_rows:
+                drows = torch.zeros(T, cfg.hidden, dtype=torch.float32, device=self.device)
+                ops.embedding_bwd_owned_(tok, g, owner, drows)
+                eng.update_token_rows(self.embed, owner, tok, drows)
+            else:
+                dtable = torch.zeros(self.embed.padded, dtype=torch.float32, device=self.device)
+                ops.embedding_bwd_(tok, g, dtable[: cfg.vocab * cfg.hidden].view(cfg.vocab, cfg.hidden))
+                eng.reduce_and_step(self.embed, fp32_full_grad=dtable)
             eng.prefetch(self.embed)  # next step starts with it
             eng.finish_step()
             if return_loss:

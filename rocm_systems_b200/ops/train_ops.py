@@ -35,6 +35,9 @@ def _lib_ops():
         lib.b200ops_adamw.argtypes = [vp, vp, vp, vp, vp, ll, f32, f32, f32, f32, f32, i32, f32, vp]
         lib.b200ops_embedding_fwd.argtypes = [vp, vp, vp, ll, i32, vp]
         lib.b200ops_embedding_bwd.argtypes = [vp, vp, vp, ll, i32, vp]
+        lib.b200ops_embedding_owner.argtypes = [vp, vp, ll, ll, vp]
+        lib.b200ops_embedding_bwd_owned.argtypes = [vp, vp, vp, vp, ll, i32, vp]
+        lib.b200ops_adamw_rows.argtypes = [vp] * 7 + [ll, i32] + [f32] * 5 + [i32, vp]
         lib.b200ops_cast_scale.argtypes = [vp, vp, ll, f32, i32, vp]
         _sigs_done = True
     return lib
@@ -202,6 +205,34 @@ def embedding_bwd_(tokens: torch.Tensor, dout: torch.Tensor, dtable_f32: torch.T
     dout = _bf16c(dout)
     H = dtable_f32.shape[1]
     _ck(_lib_ops().b200ops_embedding_bwd(tokens.contiguous().data_ptr(), dout.data_ptr(), dtable_f32.data_ptr(), tokens.numel(), H, _s()), "embedding_bwd")
+
+
+def embedding_owner(tokens: torch.Tensor, vocab: int) -> torch.Tensor:
+    """int32 [vocab]: the index of the first of ``tokens`` with that id, 0x7f7f7f7f for ids that no token has."""
+    assert tokens.dtype == torch.int64
+    owner = torch.empty(vocab, dtype=torch.int32, device=tokens.device)
+    tokens = tokens.contiguous()
+    _ck(_lib_ops().b200ops_embedding_owner(tokens.data_ptr(), owner.data_ptr(), tokens.numel(), vocab, _s()), "embedding_owner")
+    return owner
+
+
+def embedding_bwd_owned_(tokens: torch.Tensor, dout: torch.Tensor, owner: torch.Tensor, drows_f32: torch.Tensor) -> None:
+    """``embedding_bwd_`` into a compact [tokens, H] buffer: the gradient of an id's row is summed in the row of the token that owns it."""
+    dout = _bf16c(dout)
+    assert drows_f32.dtype == torch.float32 and drows_f32.is_contiguous() and drows_f32.shape == (tokens.numel(), dout.shape[-1])
+    _ck(_lib_ops().b200ops_embedding_bwd_owned(tokens.contiguous().data_ptr(), dout.data_ptr(), drows_f32.data_ptr(), owner.data_ptr(), tokens.numel(),
+                                               drows_f32.shape[1], _s()), "embedding_bwd_owned")
+
+
+def adamw_rows_(master, m, v, param, owner, hidden, lr, betas, eps, weight_decay, step, tokens=None, drows=None) -> None:
+    """AdamW on the rows of a flat [vocab * hidden] table that no token has (gradient zero), or with ``tokens`` and ``drows``
+    on the rows that one of the tokens owns."""
+    rows = owner.numel() if tokens is None else tokens.numel()
+    assert master.dtype == torch.float32 and param.dtype == torch.bfloat16 and min(t.numel() for t in (master, m, v, param)) >= owner.numel() * hidden
+    tokens = None if tokens is None else tokens.contiguous()
+    _ck(_lib_ops().b200ops_adamw_rows(master.data_ptr(), m.data_ptr(), v.data_ptr(), None if drows is None else drows.data_ptr(), param.data_ptr(), owner.data_ptr(),
+                                      None if tokens is None else tokens.data_ptr(), rows, hidden, lr, betas[0], betas[1], eps, weight_decay, step, _s()),
+        "adamw_rows")
 
 
 def cast_scale_(src_bf16: torch.Tensor, dst_f32: torch.Tensor, scale: float, accumulate: bool = False) -> None:

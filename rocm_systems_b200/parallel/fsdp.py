@@ -290,6 +290,29 @@ class FSDPEngine:
         unit.full_grad = None
         self._pending.append(done)
 
+    @property
+    def updates_rows(self) -> bool:
+        """Whether a table's rows can be updated on their own (``update_*_rows``): nothing is reduced over ranks and no update
+        waits for the norm of all gradients."""
+        return self.world == 1 and self.opt.max_grad_norm is None
+
+    def update_idle_rows(self, unit: FlatUnit, owner: torch.Tensor, hidden: int) -> None:
+        """AdamW, on the communication stream, of the rows of ``unit``'s table without a token in the batch (``owner`` from
+        ``ops.embedding_owner``). Their gradient is zero and the step reads none of them, so this may run beside its backward pass."""
+        o = self.opt
+        self.comm_stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(self.comm_stream):
+            ops.adamw_rows_(unit.master, unit.m, unit.v, unit.shard, owner, hidden, o.lr, o.betas, o.eps, o.weight_decay, self.step_count + 1)
+            done = torch.cuda.Event()
+            done.record(self.comm_stream)
+        owner.record_stream(self.comm_stream)
+        self._pending.append(done)
+
+    def update_token_rows(self, unit: FlatUnit, owner: torch.Tensor, tokens: torch.Tensor, drows: torch.Tensor) -> None:
+        """The other rows, on the current stream, with their gradients in ``drows`` (``ops.embedding_bwd_owned_``)."""
+        o = self.opt
+        ops.adamw_rows_(unit.master, unit.m, unit.v, unit.shard, owner, drows.shape[1], o.lr, o.betas, o.eps, o.weight_decay, self.step_count + 1, tokens, drows)
+
     def _clip_and_update(self) -> None:
         """With ``max_grad_norm``: sum the squared norms over the ranks, scale every held gradient shard by
         ``min(1, max_norm / norm)`` on the device (no host round trip) and run the deferred AdamW updates."""
