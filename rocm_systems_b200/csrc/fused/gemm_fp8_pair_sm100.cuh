@@ -70,6 +70,10 @@ __device__ __forceinline__ void gemmFp8PairCta(const Params& p, uint8_t* smemRaw
   const uint32_t cr = clusterCtaRank();
   volatile int* err = p.err;
 
+  if constexpr (GROUPED) {  // the counts are read side by side, then summed
+    for (int g = threadIdx.x; g <= p.groups; g += kThreads) prefix[g] = g == 0 ? 0 : (min((int)p.cnt[g - 1], p.cap) + BT - 1) / BT;
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
     prefetchTensorMap(&p.mapA);
     prefetchTensorMap(&p.mapB);
@@ -79,14 +83,8 @@ __device__ __forceinline__ void gemmFp8PairCta(const Params& p, uint8_t* smemRaw
     }
     for (int b = 0; b < kAccBufs; b++) mbarInit(&accEmpty[b], 16);
     fenceBarrierInit();
-    if constexpr (GROUPED) {
-      int acc = 0;
-      for (int g = 0; g < p.groups; g++) {
-        prefix[g] = acc;
-        acc += (min((int)p.cnt[g], p.cap) + BT - 1) / BT;
-      }
-      prefix[p.groups] = acc;
-    }
+    if constexpr (GROUPED)
+      for (int g = 0; g < p.groups; g++) prefix[g + 1] += prefix[g];
   }
   if (warp == 1) {
     tmemAllocPair(tmemSlot, kTmemCols);

@@ -129,6 +129,10 @@ __device__ __forceinline__ void gemmPairCta(const Params& p, uint8_t* smemRaw) {
   const uint32_t cr = clusterCtaRank();  // 0: issues the MMAs; 1: its partner
   volatile int* err = p.err;
 
+  if constexpr (MODE == kRows) {  // the counts are read side by side, then summed
+    for (int g = threadIdx.x; g <= p.groups; g += kThreads) prefix[g] = g == 0 ? 0 : (min((int)p.cnt[g - 1], p.cap) + 2 * BM - 1) / (2 * BM);
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
     prefetchTensorMap(&p.mapA);
     prefetchTensorMap(&p.mapB);
@@ -141,14 +145,8 @@ __device__ __forceinline__ void gemmPairCta(const Params& p, uint8_t* smemRaw) {
       mbarInit(&accEmpty[b], 8);  // four epilogue warps in each CTA of the pair
     }
     fenceBarrierInit();
-    if constexpr (MODE == kRows) {
-      int acc = 0;
-      for (int g = 0; g < p.groups; g++) {
-        prefix[g] = acc;
-        acc += (min((int)p.cnt[g], p.cap) + 2 * BM - 1) / (2 * BM);
-      }
-      prefix[p.groups] = acc;
-    }
+    if constexpr (MODE == kRows)
+      for (int g = 0; g < p.groups; g++) prefix[g + 1] += prefix[g];
   }
   if (warp == 1) {
     tmemAllocPair(tmemSlot, C::kTmemCols);
