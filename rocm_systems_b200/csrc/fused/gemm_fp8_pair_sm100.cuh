@@ -8,6 +8,9 @@
 // and the eight epilogue warps of each CTA have one block's MMA time to fold a block: 128 columns per thread, the next
 // block's scales already loaded, the buffer given back before the last FMAs.
 //
+// Bound by that fold: 4096 x 8192 x 4096 takes 184 us, 135 without the FMAs (packed two to an instruction they took 207, as they cost moves
+// and spills); 4096 x 28672 x 4096 551 us = 1.75 PFLOP/s, 622 on the one-CTA kernel.
+//
 // Warp 0 of each CTA loads its 128 rows of A and its half of B's 256 rows, the even CTA's warp 1 issues the MMAs, and one commit per
 // block, addressed to both CTAs, says that the stage is free AND the product is ready. Every wait is bounded.
 //
