@@ -119,6 +119,33 @@ def test_quantiser_codes_are_those_of_an_ieee_division(size):
         assert torch.equal(got[0].view(torch.uint8)[ok], want[0].view(torch.uint8)[ok]) and torch.equal(got[1], want[1])
 
 
+@pytest.mark.parametrize("amax", [0.0, 2.0 ** -133, 1e-20, 1.0, 3e38])
+def test_quantisers_keep_the_sign_of_zeros_and_of_what_rounds_to_zero(amax):
+    """-0, the smallest negative numbers and quotients below half a code step become the code 0x80 as they do in a division; the expert layer's
+    dispatch quantises the same way (its bf16 copy of the rows holds -0 there). Whole codes are compared."""
+    from rocm_systems_b200.comm import Communicator, get_unique_id
+    from rocm_systems_b200.ops import fp8
+    from rocm_systems_b200.parallel.ep import MoELayer, dequantize_e4m3_per128, quantize_e4m3_per128
+
+    E, H = 32, 1024
+    g = torch.Generator(device="cuda").manual_seed(3)
+    small = torch.tensor([-0.0, 0.0, -(2.0 ** -133), 2.0 ** -133, -(2.0 ** -126), 2.0 ** -126, -1e-30, 1e-30], device="cuda")
+    x = small[torch.randint(0, len(small), (E, H), device="cuda", generator=g)].to(torch.bfloat16)
+    x[:, ::128] = amax
+    x[1::2, ::128] = -amax
+    assert bool((x.view(torch.int16) == -32768).any())      # -0 is in there
+    for got, want in ((fp8.quantize_act(x), fp8.ref_quantize_act(x)), (fp8.quantize_weight(x), fp8.ref_quantize_weight(x))):
+        assert torch.equal(got[0].view(torch.uint8), want[0].view(torch.uint8)) and torch.equal(got[1], want[1])
+    comm = Communicator(0, 1, get_unique_id(), 0)
+    moe = MoELayer(comm, E, H, 128, 1, E, capacity=128, seed=5)
+    moe.forward(x, 4.0 * torch.eye(E, device="cuda"))       # token e is the one row of expert e
+    rows = moe.xb.view(E, 128, H)[:, 0]
+    torch.cuda.synchronize()
+    assert torch.equal(rows.view(torch.int16), dequantize_e4m3_per128(*quantize_e4m3_per128(x)).view(torch.int16))
+    moe.free()
+    comm.destroy()
+
+
 @pytest.mark.parametrize("M,N,K", [(1000, 8200, 1152), (129, 28680, 1152), (513, 8192, 1152), (2049, 8200, 640), (4096, 6144, 512), (4097, 4104, 512)])
 def test_fp8_gemm_on_cta_pairs_equals_the_one_cta_kernel(M, N, K):
     """Sizes that the rule sends to CTA pairs (ragged rows, columns and an odd number of blocks of K): every partial product is folded in the
