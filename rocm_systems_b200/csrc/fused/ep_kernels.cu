@@ -18,6 +18,7 @@
 // Receive buffers and counters are double buffered by call parity; counters of the other parity
 // are cleared by the dispatch that does not use them.
 #include <algorithm>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 
@@ -559,6 +560,14 @@ ncclResult_t checkShape(int expertsLocal, int cap, int hidden, int ffn, int k) {
   return ncclSuccess;
 }
 
+// All of them 16-byte aligned, which the kernels' wide accesses and the tensor maps need. Asked before the first of several launches, as a
+// later one's refusal would come too late.
+bool aligned16(std::initializer_list<const void*> ptrs) {
+  for (const void* p : ptrs)
+    if ((uintptr_t)p & 15) return false;
+  return true;
+}
+
 // What the launches behind a dispatch need to know about it.
 struct Arrived {
   EpLayout L;
@@ -663,6 +672,7 @@ static ncclResult_t epExperts(const char* what, ncclComm_t comm, void* winSym, c
   BCHECK(commCheck(c));
   BCHECK(checkShape(expertsLocal, cap, hidden, ffn, 1));
   if (!winSym || !w13 || !w2 || (!fp8 && !xb) || !act) BFAIL(ncclInvalidArgument, "%s: null buffer", what);
+  if (!aligned16({winSym, w13, w2, xb, act})) BFAIL(ncclInvalidArgument, "%s: misaligned operands", what);
   EpGuard g(c->cudaDev);
   Arrived a;
   BCHECK(arrived(what, c, winSym, expertsLocal, cap, hidden, ffn, &a));
@@ -750,6 +760,7 @@ ncclResult_t b200collEpExpertsBackward(ncclComm_t comm, void* winSym, const void
   BCHECK(commCheck(c));
   BCHECK(checkShape(expertsLocal, cap, hidden, ffn, 1));
   if (!winSym || !dOut || !w13 || !w2 || !xb || !act || !gu || !dAct || !dW13 || !dW2) BFAIL(ncclInvalidArgument, "b200collEpExpertsBackward: null buffer");
+  if (!aligned16({winSym, dOut, w13, w2, xb, act, gu, dAct, dW13, dW2})) BFAIL(ncclInvalidArgument, "b200collEpExpertsBackward: misaligned operands");
   EpGuard g(c->cudaDev);
   Arrived a;
   BCHECK(arrived("b200collEpExpertsBackward", c, winSym, expertsLocal, cap, hidden, ffn, &a));
@@ -786,6 +797,7 @@ ncclResult_t b200collEpGateGrad(ncclComm_t comm, void* winSym, const void* dy, c
   BCHECK(commCheck(c));
   BCHECK(checkShape(expertsLocal, cap, hidden, ffn, k));
   if (!winSym || !dy || !topIdx || !sentSlot || !dGate) BFAIL(ncclInvalidArgument, "b200collEpGateGrad: null buffer");
+  if (!aligned16({winSym, dy})) BFAIL(ncclInvalidArgument, "b200collEpGateGrad: misaligned operands");
   EpGuard g(c->cudaDev);
   GateGradArgs a{};
   a.L = makeLayout(c->nranks, expertsLocal, cap, hidden, ffn);
@@ -807,6 +819,7 @@ ncclResult_t b200collEpGatherGrad(ncclComm_t comm, void* winSym, const void* dyS
   BCHECK(commCheck(c));
   BCHECK(checkShape(expertsLocal, cap, hidden, ffn, k));
   if (!winSym || !dySym || !gateSym || !dOut) BFAIL(ncclInvalidArgument, "b200collEpGatherGrad: null buffer");
+  if (!aligned16({winSym, dySym, dOut})) BFAIL(ncclInvalidArgument, "b200collEpGatherGrad: misaligned operands");
   EpGuard g(c->cudaDev);
   GatherGradArgs a{};
   a.L = makeLayout(c->nranks, expertsLocal, cap, hidden, ffn);

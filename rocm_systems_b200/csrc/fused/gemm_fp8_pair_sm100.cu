@@ -49,6 +49,7 @@ bool prefersPair(int M, int N, int K) {
 // rows in turn, N is a multiple of 128.
 cudaError_t gemmFp8Pair(const void* A8, const float* sA, size_t sABlock, size_t sARow, const void* B8, const float* sB, void* C, int M, int N, int K, int lda,
                         int ldb, int ldc, bool swiglu, cudaStream_t s) {
+  if ((reinterpret_cast<uintptr_t>(C) & 15) || (ldc & 7)) return cudaErrorInvalidValue;  // rows of C are written in 16-byte pieces
   Params p{};
   if (!gemm::makeTileMap(&p.mapA, A8, M, K, lda, 128, 1) || !gemm::makeTileMap(&p.mapB, B8, N, K, ldb, 128, 1)) return cudaErrorInvalidValue;
   p.sA = sA;
@@ -72,6 +73,7 @@ cudaError_t gemmFp8Pair(const void* A8, const float* sA, size_t sABlock, size_t 
 // 64 gate and 64 up rows in turn, N % 256 == 0.
 cudaError_t gemmFp8PairGroupedSwiglu(const void* A8, const float* sA, const void* B8, const float* sB, void* C, const uint32_t* cnt, int groups, int cap, int N, int K,
                                      cudaStream_t s) {
+  if (reinterpret_cast<uintptr_t>(C) & 15) return cudaErrorInvalidValue;
   Params p{};
   if (groups > kMaxGroups || N % BT || !gemm::makeTileMap(&p.mapA, A8, (uint64_t)groups * cap, K, K, 128, 1) ||
       !gemm::makeTileMap(&p.mapB, B8, (uint64_t)groups * N, K, K, 128, 1))

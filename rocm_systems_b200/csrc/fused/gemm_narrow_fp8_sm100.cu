@@ -69,6 +69,7 @@ bool prefersNarrow(int M, int N, int K) {
 // quantiser of X, launched without the early start itself, and lets this one begin before it ends.
 cudaError_t gemmNarrowFp8(const void* X8, const float* sX, size_t sXBlock, size_t sXRow, const void* W8, const float* sW, void* C, int M, int N, int K, int ldx,
                           int ldw, int ldc, bool swiglu, bool early, cudaStream_t s) {
+  if ((reinterpret_cast<uintptr_t>(C) & 15) || (ldc & 7)) return cudaErrorInvalidValue;
   Params p{};
   p.sX = sX;
   p.sXBlock = sXBlock;
@@ -93,6 +94,7 @@ cudaError_t gemmNarrowFp8(const void* X8, const float* sX, size_t sXBlock, size_
 // sX [groups * cap][K / 128], N % 128 == 0, K at most kMaxBlocks blocks.
 cudaError_t gemmNarrowGroupedFp8(const void* X8, const float* sX, const void* W8, const float* sW, void* C, const uint32_t* cnt, int groups, int cap, int avg, int N,
                                  int K, bool swiglu, cudaStream_t s) {
+  if (reinterpret_cast<uintptr_t>(C) & 15) return cudaErrorInvalidValue;
   Params p{};
   p.sX = sX;
   p.sXBlock = 1;

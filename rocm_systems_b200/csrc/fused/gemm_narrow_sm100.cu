@@ -70,6 +70,7 @@ int splitsFor(int tiles, int tokTiles, int kSteps) {
 namespace {
 
 cudaError_t run(Params& p, const void* X, const void* W, int xRows, int groups, int tn, int ldx, int ldw, bool wMn, cudaStream_t s) {
+  if ((reinterpret_cast<uintptr_t>(p.C) & 15) || (p.ldc & 7)) return cudaErrorInvalidValue;  // as for the CTA-pair kernel, which stores wider pieces
   const bool okW = wMn ? gemm::makeTileMap(&p.mapW, W, (uint64_t)groups * p.K, p.N, ldw, 64, 2) : gemm::makeTileMap(&p.mapW, W, (uint64_t)groups * p.N, p.K, ldw, 64, 2);
   if (!okW || !gemm::makeTileMap(&p.mapX, X, xRows, p.K, ldx, tn, 2)) return cudaErrorInvalidValue;
   p.err = gemm::errWord();

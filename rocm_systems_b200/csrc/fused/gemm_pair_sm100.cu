@@ -117,11 +117,13 @@ cudaError_t gemmPairSwiglu(const void* A, const void* W, void* C, int M, int N, 
 // C [groups * cap, N or N / 2] = A [groups * cap, K] * W_g^T over the first cnt[g] rows of every group. wMn: W_g is stored [K, N] (K a
 // multiple of 128), else [N, K]. swiglu: gate and up rows in turn per 128, N % 256 == 0.
 cudaError_t gemmPairGroupedRows(const void* A, const void* W, void* C, const uint32_t* cnt, int groups, int cap, int N, int K, bool wMn, bool swiglu, cudaStream_t s) {
+  if (reinterpret_cast<uintptr_t>(C) & 15) return cudaErrorInvalidValue;  // rows of C are written in 16-byte pieces
   Params p{};
   const bool okB = wMn ? gemm::makeTileMap(&p.mapB, W, (uint64_t)groups * K, N, N, 64, 2) : gemm::makeTileMap(&p.mapB, W, (uint64_t)groups * N, K, K, 128, 2);
   if (!okB || !gemm::makeTileMap(&p.mapA, A, (uint64_t)groups * cap, K, K, BM, 2) || groups > kMaxGroups || (wMn && (swiglu || K % 128))) return cudaErrorInvalidValue;
   p.C = (__nv_bfloat16*)C;
   p.ldc = swiglu ? N / 2 : N;
+  if (p.ldc & 7) return cudaErrorInvalidValue;
   p.N = N;
   p.K = K;
   p.tilesN = (N + 255) / 256;
@@ -138,6 +140,7 @@ cudaError_t gemmPairGroupedRows(const void* A, const void* W, void* C, const uin
 // C [groups * M, N]: C_g = A[rows of g]^T * B[rows of g], A [groups * cap, M], B [groups * cap, N]; rows from cnt[g] to the next multiple
 // of 16 are zeros in both.
 cudaError_t gemmPairGroupedSum(const void* A, const void* B, void* C, const uint32_t* cnt, int groups, int cap, int M, int N, cudaStream_t s) {
+  if ((reinterpret_cast<uintptr_t>(C) & 15) || (N & 7)) return cudaErrorInvalidValue;
   Params p{};
   if (!gemm::makeTileMap(&p.mapA, A, (uint64_t)groups * cap, M, M, 64, 2) || !gemm::makeTileMap(&p.mapB, B, (uint64_t)groups * cap, N, N, 64, 2))
     return cudaErrorInvalidValue;
