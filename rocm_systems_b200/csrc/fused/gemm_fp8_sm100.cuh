@@ -67,8 +67,9 @@ struct Params {
 // division per element: with r = RN(1 / scale) and q0 = RN(x r), q = RN(q0 + r (x - q0 scale)) is the correctly rounded quotient
 // (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990, theorem on division with a
 // correctly rounded reciprocal) as long as nothing underflows: the scale is at least 1e-10 / 448, so a quotient that does not round
-// to the code 0 has a remainder far above the smallest normal number. A remainder of zero leaves q0, which is exact then and, for x = -0,
-// carries the sign that adding +0 would lose. A scale that is not finite takes the division itself.
+// to the code 0 has a remainder far above the smallest normal number. The remainder is computed negated, q0 scale - x, so that where it is
+// zero the correction adds -0, which leaves q0 and with it the sign of x = -0 (a select on the remainder does the same but
+// costs: fp8.linear of 32 x 14336 26.4 - 26.6 us in place of 24.1 - 25.5). A scale that is not finite takes the division itself.
 struct QuantScale {
   float scale, recip;
   __device__ __forceinline__ explicit QuantScale(float amax) {
@@ -77,8 +78,7 @@ struct QuantScale {
   }
   __device__ __forceinline__ float div(float x) const {
     const float q = x * recip;
-    const float rem = fmaf(-q, scale, x);
-    const float r = rem == 0.f ? q : fmaf(rem, recip, q);
+    const float r = fmaf(-fmaf(q, scale, -x), recip, q);
     return recip != 0.f ? r : __fdiv_rn(x, scale);
   }
   // 8 bf16 values -> 8 codes
