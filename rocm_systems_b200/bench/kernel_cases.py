@@ -8,7 +8,8 @@ Cases (inputs are larger than the 126 MB L2 where the kernel streams memory, and
     gemm        the CTA-pair tcgen05 GEMM in its three operand orders and the one-CTA kernel, 4096 x 4096 x 4096
     fp8         block-scaled e4m3 GEMM and its two quantisers, 4096 x 4096 x 4096
     tp          fused all-gather->GEMM(+SwiGLU) and GEMM->reduce-scatter on a communicator of one rank (tiles, policies,
-                epilogues, staging and reducer run as on many ranks; nothing crosses a link)
+                epilogues, staging and reducer run as on many ranks; nothing crosses a link). One rank on its own takes the
+                plain GEMMs instead, so this case sets B200COLL_FUSED_ONE_RANK=1 unless the environment says otherwise
     ep          expert-parallel route / dispatch / grouped expert GEMMs / combine on one rank (32 experts)
     train       RMSNorm forward + backward, RoPE, SwiGLU forward + backward, cross-entropy, embedding, AdamW at the shapes
                 of the 8B model's step
@@ -85,6 +86,7 @@ def _solo_comm():
 
 
 def case_tp(iters: int) -> dict:
+    os.environ.setdefault("B200COLL_FUSED_ONE_RANK", "1")     # read when the library is first used
     from ..ops import train_ops as ops
     from ..parallel.tp import TensorParallelMLP, TensorParallelMLPFp8
 

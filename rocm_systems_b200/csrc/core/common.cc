@@ -100,6 +100,7 @@ static void load(Flags& f) {
   if (const char* v = envOf("PIPELINE_CHUNK", false)) f.pipeChunkBytes = (long long)parseSize(v, 0);
   f.dmaGang = parseInt(envOf("DMA_GANG", false), f.dmaGang);
   f.emulateRanks = parseInt(envOf("EMULATE_RANKS", false), f.emulateRanks);
+  f.fusedOneRank = parseInt(envOf("FUSED_ONE_RANK", false), f.fusedOneRank);
   f.waitTimeoutMs = parseInt(envOf("WAIT_TIMEOUT_MS", false), f.waitTimeoutMs);
   f.bootTimeoutMs = parseInt(envOf("BOOTSTRAP_TIMEOUT_MS", false), f.bootTimeoutMs);
   if (const char* v = envOf("COMM_ID")) f.commId = v;
@@ -263,6 +264,8 @@ const SettingDoc kSettings[] = {
     {"DMA_GANG", false, "0", "copy engines one copy-engine put/get is split over (0: 1, 2 or 4 by size; at most 8)"},
     {"CHECK_SYMMETRIC", false, "0", "1: before a collective takes the zero-copy path the ranks compare, over the rendezvous network, which window and offset "
                                    "each of them passed; on any difference all of them stage instead (a host exchange per call: for debugging)"},
+    {"FUSED_ONE_RANK", false, "0", "1: a communicator of one rank runs the fused tensor-parallel kernels (tile policies, staging, reducer) where it would call the "
+                                  "plain GEMMs (tests and profiling on one GPU)"},
     {"EMULATE_RANKS", false, "0", "1: ranks may share a GPU; their communicators serve only the b200collEmu* entry points, which play all ranks in one kernel (tests)"},
     {"WAIT_TIMEOUT_MS", false, "20000", "budget of every device-side wait; on expiry the kernel records the wait and returns"},
     {"BOOTSTRAP_TIMEOUT_MS", false, "120000", "budget of the host rendezvous"},
@@ -294,6 +297,7 @@ std::string currentValue(const Flags& f, const std::string& n) {
   if (n == "PIPELINE_CHUNK") return num(f.pipeChunkBytes);
   if (n == "DMA_GANG") return num(f.dmaGang);
   if (n == "EMULATE_RANKS") return num(f.emulateRanks);
+  if (n == "FUSED_ONE_RANK") return num(f.fusedOneRank);
   if (n == "CHECK_SYMMETRIC") return num(f.checkSymmetric);
   if (n == "WAIT_TIMEOUT_MS") return num(f.waitTimeoutMs);
   if (n == "BOOTSTRAP_TIMEOUT_MS") return num(f.bootTimeoutMs);

@@ -325,7 +325,7 @@ ncclResult_t b200collAgGemm(ncclComm_t comm, void* xSym, const void* w, void* ou
   // kernel (4096 x 4096 x 6144: 0.14 ms against 0.16 for the one-CTA kernel below); with it the few-row kernel, whose rule
   // says where (128 x 28672 x 4096: 47 us against 49.5, and half the device stays idle on smaller weights), else CTA pairs if
   // gate and up rows take turns per 128.
-  if (n == 1 && (!swiglu || bn == 256 || gemmn::prefersNarrow(M, wRows))) {
+  if (plainOnOneRank(n) && (!swiglu || bn == 256 || gemmn::prefersNarrow(M, wRows))) {
     cudaError_t e;
     if (!swiglu) e = gemm2::gemmPairBf16(xSym, w, out, M, wRows, K, K, K, wRows, false, false, 0, 0, stream);
     else if (gemmn::prefersNarrow(M, wRows)) e = gemmn::gemmNarrowBf16(xSym, w, out, M, wRows, K, K, K, wRows / 2, false, bn, stream);
@@ -418,7 +418,7 @@ ncclResult_t b200collGemmRs(ncclComm_t comm, const void* a_, const void* w, void
   BCHECK(rsNextCall(c, workspaceSym, bn, &calls));
   // One rank owns every row and has nobody's partial sums to add: the GEMM writes the result itself (staging and reducing a
   // single partial took 0.15 ms of 0.55 on 4096 x 4096 x 14336, and the few-row kernel splits K where 128 rows would use 16 CTAs).
-  if (n == 1) {
+  if (plainOnOneRank(n)) {
     const cudaError_t e = gemm2::gemmPairBf16(a_, w, y, M, N, K, K, K, N, false, false, 0, 0, stream);
     if (e == cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "b200collGemmRs: operands must be 16-byte aligned with rows a multiple of 16 bytes");
     if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "b200collGemmRs launch failed: %s", cudaGetErrorString(e));

@@ -113,6 +113,9 @@ __device__ __forceinline__ void reduceOwnedTiles(const RsArgs& a, int rank, int 
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------------
+// A communicator of one rank moves nothing: the plain GEMMs take its calls, unless B200COLL_FUSED_ONE_RANK asks for the
+// kernels that several ranks run (the tests and profiles of those kernels on one GPU).
+inline bool plainOnOneRank(int n) { return n == 1 && !Flags::get().fusedOneRank; }
 bool peersOf(Comm* c, const void* p, size_t bytes, char* (&out)[kMaxRanks]);
 // Flags of the all-gather side (one word per block of 128 rows, local device memory, grown on demand) and the sequence
 // number of this call on the communicator.

@@ -203,7 +203,7 @@ ncclResult_t b200collAgGemmFp8(ncclComm_t comm, void* x8Sym, float* sASym, const
   // One rank gathers nothing: the plain GEMMs take the call where their rules say so, few rows with K split over a cluster, many on CTA
   // pairs (8192 x 7168 x 8192 with SwiGLU: 0.59 ms against 0.69 for the kernel below).
   const bool narrow = gemmn8::prefersNarrow(M, wRows, K);
-  if (n == 1 && (narrow || gemm8p::prefersPair(M, wRows, K))) {
+  if (tp::plainOnOneRank(n) && (narrow || gemm8p::prefersPair(M, wRows, K))) {
     const int nOut = swiglu ? wRows / 2 : wRows;
     cudaError_t e;
     if (narrow) e = gemmn8::gemmNarrowFp8(x8Sym, sASym, (size_t)M, 1, w8, sW, out, M, wRows, K, K, K, nOut, swiglu != 0, false, stream);
@@ -299,7 +299,7 @@ ncclResult_t b200collGemmRsFp8(ncclComm_t comm, const void* a8, const float* sA,
   const size_t flags = (wsBytes - 2 * stage) / 2;
   unsigned long long calls;
   BCHECK(tp::rsNextCall(c, workspaceSym, BN, &calls));
-  if (n == 1) {  // nobody's partial sums to add: the GEMM writes the result itself
+  if (tp::plainOnOneRank(n)) {  // nobody's partial sums to add: the GEMM writes the result itself
     const int e = b200ops_gemm_fp8_block_tn(a8, sA, w8, sW, y, M, N, K, K, K, N, 0, stream);
     if (e == (int)cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "b200collGemmRsFp8: operands must be 16-byte aligned");
     if (e) BFAIL(ncclUnhandledCudaError, "b200collGemmRsFp8 launch failed: %s", cudaGetErrorString((cudaError_t)e));

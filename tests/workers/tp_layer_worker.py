@@ -12,6 +12,7 @@ sys.path.insert(0, str(Path(__file__).resolve().parents[2]))
 
 import torch  # noqa: E402
 import torch.nn.functional as F  # noqa: E402
+from tp_worker import kernels_of  # noqa: E402
 
 from rocm_systems_b200.comm import init_from_env  # noqa: E402
 from rocm_systems_b200.ops import train_ops  # noqa: E402
@@ -82,6 +83,7 @@ def main():
     ap.add_argument("--seq", type=int, default=256)
     ap.add_argument("--comm-ctas", type=int, default=0)
     ap.add_argument("--tol", type=float, default=4e-2)
+    ap.add_argument("--expect-kernels", default="")       # comma list: names that must be among the kernels of a forward and backward pass
     ap.add_argument("--time", action="store_true")        # device time of forward + backward after the check
     ap.add_argument("--skip-check", action="store_true")
     ap.add_argument("--out", default="")
@@ -151,6 +153,9 @@ def main():
             rel[tag + "dw_o"] = close("dw_o", mod.attn.grads["w_o"], shards_att[rank]["wo"].grad, args.tol, bad)
             rel[tag + "dnorm1"] = close("dnorm1", mod.grads["norm1"], n1w.grad, args.tol, bad)
             rel[tag + "dnorm2"] = close("dnorm2", mod.grads["norm2"], n2w.grad, args.tol, bad)
+    if args.expect_kernels:
+        ran = kernels_of(lambda: (mod.forward(x), mod.backward(dy)))
+        bad += [("kernel did not run", k, sorted(ran)) for k in args.expect_kernels.split(",") if not any(k in name for name in ran)]
     if args.time and not bad:
         def dev_ms(fn, warmup=3, iters=10):
             for _ in range(warmup):

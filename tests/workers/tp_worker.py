@@ -30,6 +30,15 @@ def timed(fn, comm, warmup=3, iters=10):
     return max(float.fromhex(p.decode().strip()) for p in parts)
 
 
+def kernels_of(fn):
+    """Names of the kernels that ``fn`` launches."""
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    return {e.name for e in prof.events()}
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--rows", type=int, default=256)      # rows per rank
@@ -37,6 +46,7 @@ def main():
     ap.add_argument("--ffn", type=int, default=512)       # per rank
     ap.add_argument("--fp8", action="store_true")         # the block-scaled e4m3 form of both kernels
     ap.add_argument("--comm-ctas", type=int, default=0)   # CTAs that pull the peers' rows inside the all-gather kernel; -1: copy engines pull, no SM does
+    ap.add_argument("--expect-kernels", default="")       # comma list: names that must be among the kernels of a forward pass
     ap.add_argument("--time", action="store_true")
     ap.add_argument("--out", default="")
     args = ap.parse_args()
@@ -58,6 +68,9 @@ def main():
         scale = ref.abs().max().item()
         if not (err <= 3e-2 * scale + 1e-3):
             bad.append(("mismatch", trial, err, scale))
+    if args.expect_kernels:
+        ran = kernels_of(lambda: mlp.forward(x))
+        bad += [("kernel did not run", k, sorted(ran)) for k in args.expect_kernels.split(",") if not any(k in name for name in ran)]
     res = {"nranks": n, "rows_per_rank": args.rows, "hidden": args.hidden, "ffn_local": args.ffn, "comm_ctas": args.comm_ctas}
     if args.time and not bad:
         g = torch.Generator(device=dev).manual_seed(rank)
