@@ -274,10 +274,8 @@ class LlamaTrainer:
             logits = mm_nt(hn.detach(), w_out)
             loss_rows = ops.cross_entropy_inplace(logits, tgt, 1.0 / T)
             loss = loss_rows.mean()
-            # What no token of this batch touches of the embedding is updated beside the backward pass. On a small table the extra launches
-            # cost more than its gradient buffer (tiny model: 2.5 - 2.6 ms per step against 2.4; at 2^24 elements filling and reading
-            # that buffer takes 20 us of the device).
-            by_rows = eng.updates_rows and cfg.vocab * cfg.hidden >= 1 << 24
+            # What no token of this batch touches of the embedding is updated beside the backward pass.
+            by_rows = eng.updates_rows and cfg.vocab * cfg.hidden >= eng.rows_from
             if by_rows:
                 owner = ops.embedding_owner(tok, cfg.vocab)
                 eng.update_idle_rows(self.embed, owner, cfg.hidden)

@@ -1,4 +1,5 @@
-"""AdamW of an embedding table split into rows with and without a token, against the dense update."""
+"""AdamW of an embedding table split into rows with and without a token, against the dense update: the kernels by themselves and inside
+the training step, where the rows without a token are updated on the communication stream beside the backward pass."""
 import pytest
 import torch
 
@@ -43,3 +44,46 @@ def test_row_updates_match_the_dense_update(vocab, H, T, repeat):
         else:
             assert torch.equal(x, y)
         assert torch.equal(y[n:], start[n:])
+
+
+def _embedding_after(rows_from, batches, overlap):
+    from rocm_systems_b200.models.llama import LlamaConfig, LlamaTrainer
+    from rocm_systems_b200.parallel.fsdp import AdamWConfig
+
+    cfg = LlamaConfig.tiny(64)
+    t = LlamaTrainer(cfg, None, torch.device("cuda", 0), opt=AdamWConfig(lr=1e-2, weight_decay=0.1), seed=3, overlap=overlap)
+    assert t.engine.updates_rows
+    t.engine.rows_from = rows_from
+    losses = [t.step(tok.pin_memory(), tgt.pin_memory()) for tok, tgt in batches]
+    torch.cuda.synchronize()
+    return losses, [x.clone() for x in (t.embed.master, t.embed.m, t.embed.v, t.embed.shard)]
+
+
+@pytest.mark.parametrize("overlap", [True, False])
+def test_training_steps_with_row_updates_equal_those_with_the_dense_update(overlap):
+    """Four steps whose batches hold each id once, out of ids that come and go between the steps (a row is idle in one step and owned in the
+    next, with moments that decay and weights that decay): master, moments and bf16 weights of the embedding are bit-equal."""
+    g = torch.Generator().manual_seed(1)
+    batches = [(torch.randperm(400, generator=g)[:128].view(2, 64), torch.randint(0, 1024, (2, 64), generator=g)) for _ in range(4)]
+    assert any(set(a[0].flatten().tolist()) & set(b[0].flatten().tolist()) for a, b in zip(batches, batches[1:]))
+    dense, rows = _embedding_after(float("inf"), batches, overlap), _embedding_after(0, batches, overlap)
+    assert dense[0] == rows[0]
+    for x, y in zip(dense[1], rows[1]):
+        assert torch.equal(x, y)
+
+
+def test_a_training_step_with_repeated_ids():
+    """One step of a batch of few ids, each many times: the rows without a token are bit-equal to the dense update's, the others are rows whose
+    fp32 sums depend on the order of the atomics on both paths (bounded in the test of the kernels) and have all moved."""
+    g = torch.Generator().manual_seed(2)
+    tok = torch.randint(0, 7, (2, 64), generator=g)
+    batches = [(tok, torch.randint(0, 1024, (2, 64), generator=g))]
+    (_, dense), (_, rows) = _embedding_after(float("inf"), batches, True), _embedding_after(0, batches, True)
+    owned = torch.zeros(1024, dtype=torch.bool)
+    owned[tok.flatten().unique()] = True
+    n = 1024 * 256
+    for x, y in zip(dense, rows):
+        a, b = x[:n].view(1024, 256)[~owned.cuda()], y[:n].view(1024, 256)[~owned.cuda()]
+        assert torch.equal(a, b)
+    for x in (dense[1], rows[1]):                     # first moments
+        assert bool((x[:n].view(1024, 256)[owned.cuda()] != 0).any(1).all()) and not bool(x[:n].view(1024, 256)[~owned.cuda()].any())
