@@ -35,6 +35,7 @@ def _lib_ep():
         lib.b200collEpCounts.argtypes = [vp, vp, i32, i32, i32, i32, vp, vp, vp]
         lib.b200collEpGateGrad.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp]
         lib.b200collEpGatherGrad.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp]
+        lib.b200collEpGroupedGemm.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp]
         lib.b200collEpExpertsBackward.argtypes = [vp] * 11 + [i32] * 4 + [vp]
         lib.b200collEpRouterGrad.argtypes = [vp, vp, vp, vp, i32, i32, i32, vp]
         _done = True

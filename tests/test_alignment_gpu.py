@@ -1,6 +1,4 @@
 """Misaligned buffers of the grouped and one-rank GEMM entry points: the host refuses them, before anything is launched."""
-import ctypes
-
 import pytest
 import torch
 
@@ -58,8 +56,6 @@ def test_expert_gemms_refuse_misaligned_buffers(comm, layers):
     _refused(lib.b200collEpExpertsFp8, [h, m8._win.ptr, m8.w13_q.data_ptr(), m8.w13_s.data_ptr(), m8.w2.data_ptr(), m8.act.data_ptr(), *dims, s], (2, 4, 5))
     _refused(lib.b200collEpGatherGrad, [h, m._win.ptr, m.out.data_ptr(), m.top_w.data_ptr(), m.d_out.data_ptr(), m.T, m.k, *dims, s], (2, 4))
     _refused(lib.b200collEpGateGrad, [h, m._win.ptr, m.out.data_ptr(), m.top_idx.data_ptr(), m.sent.data_ptr(), m.d_gate.data_ptr(), m.T, m.k, *dims, s], (2,))
-    vp, i32 = ctypes.c_void_p, ctypes.c_int
-    lib.b200collEpGroupedGemm.argtypes = [vp] * 5 + [i32] * 6 + [vp]
     _refused(lib.b200collEpGroupedGemm, [h, m._win.ptr, m.d_out.data_ptr(), m.w13.data_ptr(), m.gu.data_ptr(), 2 * m.ffn, m.hidden, *dims, s], (2, 3, 4))
     torch.cuda.synchronize()
     assert ops.gemm_take_error() == 0

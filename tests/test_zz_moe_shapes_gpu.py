@@ -89,3 +89,68 @@ def test_experts_match_float64(comm, hidden, ffn, k, rows, fp8):
                 assert float((a.double() - b).norm()) <= 2.0 ** -6 * float(b.norm()), (trial, i)
     finally:
         moe.free()
+
+
+@pytest.mark.parametrize("rows", [[1, 40, 0, 128, 33], [97, 256, 0, 511, 2300]])      # few rows per expert on average, and more than 96
+@pytest.mark.parametrize("w_rows,K", [(128, 200), (384, 1000), (640, 64), (1024, 1032)])
+def test_grouped_gemm_matches_float64(comm, rows, w_rows, K):
+    """The grouped GEMM a program can call by itself, with weight rows that end inside a 256-column tile and reductions that end inside a 64-step slice.
+    Nothing is written past an expert's rows, and what lies past them in the input does not matter. 1024 weight rows: the result
+    goes to the window, where combine with unit weights finds it. Bound: the bf16 rounding of the result and one fp32 truncation per 16
+    steps of a sum that stays below the sum of magnitudes."""
+    from rocm_systems_b200 import _lib
+    from rocm_systems_b200.ops import train_ops as ops
+    from rocm_systems_b200.parallel.ep import MoELayer, _lib_ep
+
+    E, H = 32, 1024
+    counts = rows + [0] * (E - len(rows))
+    T = sum(counts)
+    moe = MoELayer(comm, E, H, 128, 1, T, capacity=max(max(counts), 128), seed=5)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(w_rows + K)
+        moe.forward(torch.randn(T, H, device="cuda", generator=g).to(torch.bfloat16), _logits(counts, E, 1))
+        assert moe.counts() == (counts, 0)
+        a = torch.randn(E, moe.cap, K, device="cuda", generator=g).to(torch.bfloat16)
+        for e in range(E):
+            a[e, counts[e]:] = float("nan")
+        w = torch.randn(E, w_rows, K, device="cuda", generator=g).to(torch.bfloat16)
+        out = torch.full((E, moe.cap, w_rows), 7.0, dtype=torch.bfloat16, device="cuda")
+        to_window = w_rows == H
+        _lib.check(_lib_ep().b200collEpGroupedGemm(comm.handle, moe._win.ptr, a.data_ptr(), w.data_ptr(), None if to_window else out.data_ptr(), w_rows, K, *moe._args(),
+                                                   ops._s()), "b200collEpGroupedGemm")
+        if to_window:
+            y, ones = torch.empty(T, H, dtype=torch.bfloat16, device="cuda"), torch.ones(T, 1, device="cuda")
+            _lib.check(_lib_ep().b200collEpCombine(comm.handle, moe._win.ptr, moe.top_idx.data_ptr(), ones.data_ptr(), moe.sent.data_ptr(), y.data_ptr(), T, 1, *moe._args(),
+                                                   ops._s()), "b200collEpCombine")
+            out[moe.top_idx[:, 0].long(), moe.sent[:, 0].long()] = y
+        torch.cuda.synchronize()
+        assert ops.gemm_take_error() == 0
+        for e in range(E):
+            x, ww, got = a[e, :counts[e]].double(), w[e].double(), out[e]
+            ref = x @ ww.t()
+            tol = ref.abs() * 2.0 ** -8 + (x.abs() @ ww.abs().t()) * 2.0 ** -23 * (K // 16 + 1)
+            assert bool(((got[:counts[e]].double() - ref).abs() <= tol).all()), e
+            assert bool((got[counts[e]:] == 7).all()), e
+    finally:
+        moe.free()
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 32, 1), (33, 32, 8), (1000, 64, 2), (9, 1024, 8), (257, 256, 5)])
+def test_router_gradient_matches_its_oracle(T, E, k):
+    """Against the formula in float64; bound: k products and sums of fp32 in the dot product, two more operations behind it."""
+    from rocm_systems_b200 import _lib
+    from rocm_systems_b200.ops import train_ops as ops
+    from rocm_systems_b200.parallel.ep import _lib_ep, router_backward
+
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    idx = torch.argsort(torch.randn(T, E, device="cuda", generator=g), dim=-1)[:, :k].to(torch.int32).contiguous()
+    w = torch.softmax(torch.randn(T, k, device="cuda", generator=g), -1)
+    d = torch.randn(T, k, device="cuda", generator=g)
+    out = torch.full((T, E), 7.0, device="cuda")
+    _lib.check(_lib_ep().b200collEpRouterGrad(w.data_ptr(), idx.data_ptr(), d.data_ptr(), out.data_ptr(), T, E, k, ops._s()), "b200collEpRouterGrad")
+    torch.cuda.synchronize()
+    ref = router_backward(w.double(), idx, d.double(), E)
+    size = (d.abs() + (d * w).abs().sum(-1, keepdim=True)).double().amax(-1, keepdim=True)
+    assert bool(((out.double() - ref).abs() <= (k + 3) * 2.0 ** -23 * size).all())
+    selected = torch.zeros(T, E, dtype=torch.bool, device="cuda").scatter_(1, idx.long(), True)
+    assert not bool(out[~selected].any())
