@@ -216,9 +216,12 @@ __device__ __forceinline__ void gemmFp8PairCta(const Params& p, uint8_t* smemRaw
         }
       }
       if (!ok) break;
+      if (row0 >= o.aEnd) continue;
       if constexpr (SWIGLU) {  // 64 gate columns, then the 64 up columns of the same outputs
+        if (live) {            // not on the zeros of rows past the end, whose division takes the slow path
 #pragma unroll
-        for (int i = 0; i < 64; i++) acc[i] = acc[i] / (1.f + __expf(-acc[i])) * acc[64 + i];
+          for (int i = 0; i < 64; i++) acc[i] = acc[i] / (1.f + __expf(-acc[i])) * acc[64 + i];
+        }
         gemm8::storeCols<64>(
             sw, lane, p.N / 2 - o.tn * (BT / 2), acc,
             [&](int r) -> __nv_bfloat16* { return row0 + r < o.aEnd ? p.C + (size_t)(row0 + r) * p.ldc + (size_t)o.tn * (BT / 2) : nullptr; },

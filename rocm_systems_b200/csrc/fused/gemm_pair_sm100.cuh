@@ -268,7 +268,10 @@ __device__ __forceinline__ void gemmPairCta(const Params& p, uint8_t* smemRaw) {
       if (!mbarWait(&accFull[b], accPhase, err, gemm::ERR_EPI_ACC_FULL)) { ok = false; break; }
       tcFenceAfter();
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN);
-      gemm::drainStaged(
+      // Rows past the end are neither read back nor run through the activation: they are zeros as a rule, and dividing zeros takes the
+      // slow path of the division (2176 x 8192 x 1024, half of the last row tile past the end: 110 us, 53 without).
+      const bool live = row0 + lane < o.cEnd;
+      if (row0 < o.cEnd) gemm::drainStaged(
           sw, lane, kOut, colLimit,
           [&](int c, uint32_t(&acc)[32]) {
             tmemLoad32(taddr + c * 32, acc);
@@ -276,10 +279,12 @@ __device__ __forceinline__ void gemmPairCta(const Params& p, uint8_t* smemRaw) {
               uint32_t up[32];
               tmemLoad32(taddr + BN / 2 + c * 32, up);
               tmemLoadWait();
+              if (live) {
 #pragma unroll
-              for (int i = 0; i < 32; i++) {
-                const float g = __uint_as_float(acc[i]);
-                acc[i] = __float_as_uint(g / (1.f + __expf(-g)) * __uint_as_float(up[i]));
+                for (int i = 0; i < 32; i++) {
+                  const float g = __uint_as_float(acc[i]);
+                  acc[i] = __float_as_uint(g / (1.f + __expf(-g)) * __uint_as_float(up[i]));
+                }
               }
             } else {
               tmemLoadWait();
