@@ -254,6 +254,79 @@ __global__ void __launch_bounds__(256) epDequant(const char* __restrict__ win, E
   }
 }
 
+// ---- first expert GEMM straight on the received fp8 rows ---------------------------------------------------------
+// The rows in the window already are what the block-scaled GEMM wants: e4m3 with one fp32 scale per row and 128
+// channels (row-major here, [row][hidden / 128]). With the experts' gate/up weight quantised per 128 x 128 block
+// (interleaved per 128 rows: 64 gate rows, then the 64 up rows of the same outputs) the dequantisation pass and its
+// bf16 copy of the activations disappear, and the larger of the two GEMMs runs at fp8 rate. Three kernels share it (see fp8Kernel):
+// this one, a CTA per 128 x 128 tile, for experts whose rows fit one such tile and would leave half of a CTA pair's tile empty.
+struct GroupPolicy8 {
+  const uint32_t* cnt;  // rows per expert (may exceed cap when rows were dropped)
+  int experts;          // local experts
+  const int* prefix;    // shared memory, filled by the kernel: row blocks with tokens before expert e; [experts] = all of them
+  int cap, capTiles;
+  int wRows;            // weight rows per expert (2 ffn)
+  const float* sA;      // [expertsLocal * cap][groups]
+  int groups;           // hidden / 128
+  __nv_bfloat16* out;   // act [expertsLocal * cap, nOut]
+  int ldo, nOut;
+  __device__ __forceinline__ int have(int e) const { return min((int)cnt[e], cap); }
+  // Tile t of the compact list: only row blocks that hold tokens are numbered, expert after expert, so every CTA of the
+  // persistent grid gets the same share of real work however unevenly the tokens fell. Indices past the end map to no tile.
+  __device__ __forceinline__ void coord(int t, int, int tilesN, int& tm, int& tn) const {
+    const int rb = t / tilesN;
+    tn = t - rb * tilesN;
+    tm = -1;
+    if (rb >= prefix[experts]) return;
+    int e = 0;
+    while (prefix[e + 1] <= rb) e++;  // prefix[] sits in shared memory: a few cycles per step
+    tm = e * capTiles + (rb - prefix[e]);
+  }
+  __device__ __forceinline__ bool valid(int tm, int) const { return tm >= 0; }
+  __device__ __forceinline__ int bRow(int tm, int tn) const { return (tm / capTiles) * wRows + tn * gemm8::BN; }
+  __device__ __forceinline__ int scaleBOff(int tm, int tn) const { return ((tm / capTiles) * (wRows / gemm8::BN) + tn) * groups; }
+  __device__ __forceinline__ bool waitTile(int, int, volatile int*) const { return true; }
+  __device__ __forceinline__ bool epiBegin(int, volatile int*) const { return true; }
+  __device__ __forceinline__ float scaleA(int kb, int row) const { return __ldg(sA + (size_t)row * groups + kb); }
+  __device__ __forceinline__ void emit(float (&acc)[gemm8::kAccCols], int tm, int tn, int q, int h, int lane, uint8_t* sw) const {
+    constexpr int H = gemm8::BN / 2;
+    const int e = tm / capTiles;
+    const int row0 = tm * gemm::BM + q * 32;
+    const int rowsHave = have(e) - (row0 - e * cap);  // rows of this warp's 32 that hold tokens
+    if (rowsHave <= 0) return;
+    // gate columns 32h .. 32h+32 of the tile in acc[0..32), the up columns of the same outputs in acc[32..64); not on the zeros of rows
+    // past the end, whose division takes the slow path
+    if (lane < rowsHave) {
+#pragma unroll
+      for (int i = 0; i < 32; i++) {
+        const float g = acc[i];
+        acc[i] = g / (1.f + __expf(-g)) * acc[32 + i];
+      }
+    }
+    gemm8::storeCols<32>(
+        sw, lane, H, acc,  // ffn is a multiple of 128: every tile has all of its 64 output columns
+        [&](int r) -> __nv_bfloat16* { return r < rowsHave ? out + (size_t)(row0 + r) * ldo + (size_t)tn * H : nullptr; }, [&](int) { return h * 32; });
+  }
+  __device__ __forceinline__ void tileDone(int, int, int, int, int) const {}
+};
+
+// Row blocks with tokens before every expert, once per CTA, into shared memory: the counts are read side by side, then summed.
+__device__ __forceinline__ void fillBlockPrefix(int* prefix, const uint32_t* cnt, int experts, int cap) {
+  for (int e = threadIdx.x; e <= experts; e += blockDim.x) prefix[e] = e == 0 ? 0 : (min((int)cnt[e - 1], cap) + gemm::BM - 1) / gemm::BM;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int e = 0; e < experts; e++) prefix[e + 1] += prefix[e];
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(gemm8::kThreads, 1) groupedGemmFp8Kernel(const __grid_constant__ gemm8::Params p, GroupPolicy8 pol) {
+  extern __shared__ uint8_t smemRaw[];
+  __shared__ int prefix[kMaxLocalExperts + 1];
+  fillBlockPrefix(prefix, pol.cnt, pol.experts, pol.cap);
+  pol.prefix = prefix;
+  gemm8::gemmFp8Cta(p, pol, blockIdx.x, gridDim.x, smemRaw);
+}
+
 // ---- combine ---------------------------------------------------------------------------------------------------
 struct CombineArgs {
   const int* topIdx;      // [T, k]
@@ -585,11 +658,39 @@ ncclResult_t arrived(const char* what, Comm* c, const void* winSym, int expertsL
   return ncclSuccess;
 }
 
-// Up to 96 rows per expert on average the kernels with output features as MMA rows are faster, above CTA pairs. 32 experts, hidden 4096,
-// ffn 1024, whole forward pass: 16 rows 207 us against 262, 96 rows 254 against 271, 128 rows level, 256 rows 398 against 360;
-// with fp8 gate/up weights 157 against 240, 225 against 245, 270 against 253, 418 against 338; forward and backward 864
-// against 964, 1007 against 1013, 1062 against 1037, 1367 against 1248.
+// bf16: up to 96 rows per expert on average the kernels with output features as MMA rows are faster, above CTA pairs. Over 32 experts of
+// 1024 x 256 to 7168 x 2048 and 64 of 2048 x 512 and 4096 x 1408, rows spread evenly and as a router spreads them: at 48 rows few rows
+// are ahead everywhere (by 3 - 25 %), at 96 by 2 - 15 % with even rows and within 8 % either way with uneven ones, at 128 pairs are ahead or
+// level, at 160 by 10 - 35 %. Forward and backward of 32 experts of 4096 x 1024: 48 rows 819 us against 872, 96 rows 918 against 902.
 bool fewRows(const Arrived& a) { return a.rowsPerExpert <= 96; }
+
+// The gate/up GEMM on fp8 rows (times with the second GEMM behind it, 32 experts, counts as a router spreads them): few rows up to 32 per
+// expert on average (32 rows of 4096 x 1024: 128 us, 149 with a CTA per tile before its epilogue skipped dead rows); a CTA per 128 x 128
+// tile up to 112, where a 256-row tile of a pair would be half padding and the few-row kernel reads the weights for
+// every 64 rows of an expert (48 rows of 4096 x 1024: 137 against 150 with few rows; 80 rows of 7168 x 2048: 363 - 410 against 478 - 498
+// and 455 on pairs); pairs above (160 rows of 4096 x 1024: 172 - 183 against 183 - 202).
+enum Fp8Kernel { kFp8FewRows, kFp8OneCta, kFp8Pair };
+Fp8Kernel fp8Kernel(const Arrived& a) { return a.rowsPerExpert <= 32 ? kFp8FewRows : a.rowsPerExpert <= 112 ? kFp8OneCta : kFp8Pair; }
+
+// act [expertsLocal * cap, N / 2] = SwiGLU over the window's e4m3 rows * w8_e^T with a CTA per 128 x 128 tile; N = 2 ffn.
+cudaError_t groupedFp8OneCta(const Arrived& a, const void* rows8, const float* scales, const void* w8, const float* sW, void* act, int N, int K, cudaStream_t s) {
+  const int rows = a.L.expertsLocal * a.L.cap;
+  gemm8::Params p{};
+  if (!gemm::makeTileMap(&p.mapA, rows8, rows, K, K, gemm::BM, 1) || !gemm::makeTileMap(&p.mapB, w8, (uint64_t)a.L.expertsLocal * N, K, K, gemm8::BN, 1))
+    return cudaErrorInvalidValue;
+  p.sA = scales;
+  p.sB = sW;
+  p.C = (__nv_bfloat16*)act;
+  p.M = rows; p.N = N; p.K = K; p.ldc = N / 2;
+  p.tilesM = rows / gemm::BM; p.tilesN = N / gemm8::BN; p.kBlocks = K / 128;
+  p.err = gemm::errWord();
+  if (!p.err) return cudaErrorMemoryAllocation;
+  const GroupPolicy8 pol{a.cnt, a.L.expertsLocal, nullptr, a.L.cap, a.L.cap / gemm::BM, N, scales, K / 128, p.C, N / 2, N / 2};
+  const cudaError_t e = cudaFuncSetAttribute(groupedGemmFp8Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm8::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  groupedGemmFp8Kernel<<<std::min(gemm::smCount(), p.tilesM * p.tilesN), gemm8::kThreads, gemm8::kSmemBytes, s>>>(p, pol);
+  return cudaGetLastError();
+}
 
 cudaError_t groupedRows(const Arrived& a, const void* x, const void* w, void* out, int N, int K, bool wMn, bool swiglu, cudaStream_t s) {
   if (fewRows(a) && (!wMn || K % 64 == 0))
@@ -682,8 +783,13 @@ static ncclResult_t epExperts(const char* what, ncclComm_t comm, void* winSym, c
     // GEMM 1: act = swiglu(dequant(rows) * dequant(w13)^T) straight on the window's e4m3 rows and scales.
     const char* rows8 = win + a.L.payloadOff;
     const float* scales = (const float*)(win + a.L.scaleOff);
-    e = fewRows(a) ? gemmn8::gemmNarrowGroupedFp8(rows8, scales, w13, w13Scales, act, a.cnt, expertsLocal, cap, a.rowsPerExpert, 2 * ffn, hidden, true, stream)
-                      : gemm8p::gemmFp8PairGroupedSwiglu(rows8, scales, w13, w13Scales, act, a.cnt, expertsLocal, cap, 2 * ffn, hidden, stream);
+    switch (fp8Kernel(a)) {
+      case kFp8FewRows:
+        e = gemmn8::gemmNarrowGroupedFp8(rows8, scales, w13, w13Scales, act, a.cnt, expertsLocal, cap, a.rowsPerExpert, 2 * ffn, hidden, true, stream);
+        break;
+      case kFp8OneCta: e = groupedFp8OneCta(a, rows8, scales, w13, w13Scales, act, 2 * ffn, hidden, stream); break;
+      default: e = gemm8p::gemmFp8PairGroupedSwiglu(rows8, scales, w13, w13Scales, act, a.cnt, expertsLocal, cap, 2 * ffn, hidden, stream);
+    }
   } else {
     epDequant<<<8 * gemm::smCount(), 256, 0, stream>>>(win, a.L, a.parity, (__nv_bfloat16*)xb);
     BCUDA(cudaGetLastError());

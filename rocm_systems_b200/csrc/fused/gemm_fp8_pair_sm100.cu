@@ -11,7 +11,7 @@ namespace {
 
 template <bool GROUPED, bool SWIGLU>
 auto pairKernel() {
-  if constexpr (GROUPED) return &ep::groupedGemmFp8Kernel;
+  if constexpr (GROUPED) return &gemmFp8PairGroupedKernel;
   else return &gemmFp8PairKernel<SWIGLU>;
 }
 

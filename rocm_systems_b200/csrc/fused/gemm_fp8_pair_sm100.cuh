@@ -249,13 +249,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmFp8
   gemmFp8PairCta<false, SWIGLU>(p, smemRaw);
 }
 
-}  // namespace gemm8p
-namespace ep {
-
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm8p::kThreads, 1) groupedGemmFp8Kernel(const __grid_constant__ gemm8p::Params p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemmFp8PairGroupedKernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smemRaw[];
-  gemm8p::gemmFp8PairCta<true, true>(p, smemRaw);
+  gemmFp8PairCta<true, true>(p, smemRaw);
 }
 
-}  // namespace ep
+}  // namespace gemm8p
 }  // namespace b200

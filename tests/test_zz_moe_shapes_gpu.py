@@ -1,5 +1,5 @@
-"""The expert GEMMs of the mixture-of-experts layer where their tiles end: few rows (features as MMA rows), many (CTA pairs), experts
-without any, one expert with all, counts around the edges of 16, 32, 64, 128 and 256 rows, forward and backward."""
+"""The expert GEMMs of the mixture-of-experts layer where their tiles end: few rows (features as MMA rows), for fp8 a middle range (a CTA
+per 128 x 128 tile), many (CTA pairs), experts without any, one expert with all, counts around the edges of 16, 32, 64, 128 and 256 rows, forward and backward."""
 import pytest
 import torch
 
@@ -34,6 +34,7 @@ CASES = [
     (1024, 256, 1, [127, 128, 129, 0, 1]),
     (1024, 640, 1, [255, 256, 257, 0, 511, 512, 513, 900]),
     (3072, 128, 2, [1000, 1000]),
+    (1024, 128, 1, [0, 127, 128, 129, 300, 1, 0, 640, 255, 256, 257, 384, 385, 1200]),     # more than 112 rows per expert on average
 ]
 
 
