@@ -23,7 +23,7 @@ cudaError_t gemmPairGroupedRows(const void* A, const void* W, void* C, const uin
 cudaError_t gemmPairGroupedSum(const void* A, const void* B, void* C, const uint32_t* cnt, int groups, int cap, int M, int N, cudaStream_t s);
 }  // namespace gemm2
 namespace gemmn {
-bool prefersNarrow(int M, int N);
+bool prefersNarrow(int M, int N, int K);
 cudaError_t gemmNarrowBf16(const void* X, const void* W, void* C, int M, int N, int K, int ldx, int ldw, int ldc, bool wMn, int gateUpTile, cudaStream_t s);
 cudaError_t gemmNarrowGroupedBf16(const void* X, const void* W, void* C, const uint32_t* cnt, int groups, int cap, int avg, int N, int K, bool wMn, int gateUpTile,
                                   cudaStream_t s);

@@ -48,23 +48,32 @@ cudaError_t dispatch(const Params& p, int tn, int tiles, int groups, int S, cuda
 
 }  // namespace
 
-// Where this kernel is the faster one, measured over M 1 .. 1024, N 1024 .. 28672, K 512 .. 14336 with the weights out of
-// the L2. Up to 128 rows everywhere (N 28672, K 4096, 128 rows: 48 us against 56 on CTA pairs; N 1024, K 512: 4 - 5 against
-// 9). Above, W is read again for every 128 rows, and it pays only while the 256 x 256 tiles would leave half of the device
-// idle: 512 x 4096 x 4096 23 us against 27, 512 x 4096 x 14336 58 against 73, but 512 x 6144 x 4096 31 against 28. Above 512
-// rows never (768 x 4096 x 4096 30 against 28).
-bool prefersNarrow(int M, int N) {
+// Where this kernel is the faster one, measured over M 1 .. 1024, N 512 .. 28672, K 512 .. 14336 with the weights out of
+// the L2. Up to 128 rows nearly everywhere (N 28672, K 4096, 128 rows: 48 us against 56 on CTA pairs; N 1024, K 512: 4 - 5 against
+// 9). Above, W is read again for every 128 rows, and it pays only while the 256 x 256 tiles would leave half of the
+// device idle: 512 x 4096 x 4096 23 us against 27, 512 x 4096 x 14336 58 against 73, but 512 x 6144 x 4096 31 against 28. Above 512
+// rows never (768 x 4096 x 4096 30 against 28). Of those tiles, more than 128 CTAs are not split along K, which pays for a short
+// reduction only (256 x 9216 x 512 9.7 us against 10.8, x 4096 32.9 against 29.6, 512 x 4608 x 4096 28.9 against 27.5), and below 1024
+// steps of K two splits of 80 CTAs or more do not (256 x 8192 x 512 11.4 against 10.7, 512 x 4096 x 768 12.1 against 11.8).
+bool prefersNarrow(int M, int N, int K) {
   if (M <= 128) return true;
   const int tiles = ((M + 255) / 256) * ((N + 255) / 256);
-  return M <= 512 && 2 * tiles <= gemm2::pairsOnDevice();
+  if (M > 512 || 2 * tiles > gemm2::pairsOnDevice()) return false;
+  const int ctas = ((M + 127) / 128) * ((N + BF - 1) / BF);
+  if (ctas > 128) return K <= 1024;
+  return K >= 1024 || ctas < 80;
 }
 
 // CTAs along K: as many as fill the device two to an SM. 4096 x 4096 on 16 rows takes 14.8 us with 2 splits, 10.8 - 11.4 with 4 - 8.
 // One token tile: at most 240 CTAs, because from 128 feature tiles up the exchange costs more than the second CTA of an SM gives
 // (16384 x 2048 on 16 rows: 15.2 us unsplit, 16.1 in two). A cluster beyond that number waits for a second wave (6144 x 4096: 13.5 us
-// with 240 CTAs, 18.6 with 288).
+// with 240 CTAs, 18.6 with 288). Up to 1024 steps of K the exchange of many or uneven parts outweighs the shorter loop: 1, 2 or 4 even
+// parts (4096 x 512 on 128 rows: 12.1 us in seven, 10.4 on CTA pairs, 8.1 in four; 8192 x 1024 on 64 rows 10.7 in three, 9.7 in two),
+// except where a dozen tiles leave most of the device free (512 x 1024 on one row: 4.4 us in eight, 4.9 in four).
 int splitsFor(int tiles, int tokTiles, int kSteps) {
-  return std::max(1, std::min({kMaxSplit, kSteps, (tokTiles == 1 ? 240 : 256) / (tiles * tokTiles)}));
+  const int S = std::max(1, std::min({kMaxSplit, kSteps, (tokTiles == 1 ? 240 : 256) / (tiles * tokTiles)}));
+  if (kSteps > 16 || tiles * tokTiles <= 12) return S;
+  return S >= 4 ? 4 : S >= 2 ? 2 : 1;
 }
 
 namespace {

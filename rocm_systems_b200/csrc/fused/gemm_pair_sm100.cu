@@ -77,7 +77,7 @@ cudaError_t gemmPairBf16(const void* A, const void* B, void* C, int M, int N, in
                          cudaStream_t s) {
   if (M <= 0 || N <= 0 || K <= 0) return cudaSuccess;
   if ((reinterpret_cast<uintptr_t>(C) & 15) || (ldc & 7)) return cudaErrorInvalidValue;  // rows of C are written in 16-byte pieces
-  if (bn == 0 && maxCtas == 0 && !aMn && gemmn::prefersNarrow(M, N)) return gemmn::gemmNarrowBf16(A, B, C, M, N, K, lda, ldb, ldc, bMn, 0, s);
+  if (bn == 0 && maxCtas == 0 && !aMn && gemmn::prefersNarrow(M, N, K)) return gemmn::gemmNarrowBf16(A, B, C, M, N, K, lda, ldb, ldc, bMn, 0, s);
   // 256-wide tiles unless the caller says otherwise: on 128-wide ones the issuing thread's per-stage work (barrier wait,
   // descriptors, commit) is no longer hidden behind the MMAs, and the kernel ran 1.6x slower on the same problem.
   if (bn != 128 && bn != 256) bn = N > 128 ? 256 : 128;

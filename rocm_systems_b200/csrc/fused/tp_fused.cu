@@ -325,10 +325,10 @@ ncclResult_t b200collAgGemm(ncclComm_t comm, void* xSym, const void* w, void* ou
   // kernel (4096 x 4096 x 6144: 0.14 ms against 0.16 for the one-CTA kernel below); with it the few-row kernel, whose rule
   // says where (128 x 28672 x 4096: 47 us against 49.5, and half the device stays idle on smaller weights), else CTA pairs if
   // gate and up rows take turns per 128.
-  if (plainOnOneRank(n) && (!swiglu || bn == 256 || gemmn::prefersNarrow(M, wRows))) {
+  if (plainOnOneRank(n) && (!swiglu || bn == 256 || gemmn::prefersNarrow(M, wRows, K))) {
     cudaError_t e;
     if (!swiglu) e = gemm2::gemmPairBf16(xSym, w, out, M, wRows, K, K, K, wRows, false, false, 0, 0, stream);
-    else if (gemmn::prefersNarrow(M, wRows)) e = gemmn::gemmNarrowBf16(xSym, w, out, M, wRows, K, K, K, wRows / 2, false, bn, stream);
+    else if (gemmn::prefersNarrow(M, wRows, K)) e = gemmn::gemmNarrowBf16(xSym, w, out, M, wRows, K, K, K, wRows / 2, false, bn, stream);
     else e = gemm2::gemmPairSwiglu(xSym, w, out, M, wRows, K, stream);
     if (e == cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "b200collAgGemm: operands must be 16-byte aligned with rows a multiple of 16 bytes");
     if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "b200collAgGemm launch failed: %s", cudaGetErrorString(e));
