@@ -33,16 +33,16 @@ cudaError_t launch(const Params& p, int tiles, cudaStream_t s) {
 
 }  // namespace
 
-// Where pairs are faster than one CTA per 128 x 128 tile, from a sweep of M 136 .. 4096, N 512 .. 28672, K 512 .. 8192: a round of pairs
-// (one 256 x 256 tile each) takes 1.3 - 1.5 times as long as a round of single CTAs, so they win where they need at most two thirds of
-// the rounds. 4096 x 28672 x 8192: 1.09 ms against 1.39; 512 x 8192 x 8192 (one round against two): 53 us against 64;
-// but 384 x 28672 x 8192 (four against five) 176 against 137 and 2048 x 1024 x 8192 (one against one) 50 against 39. A short
+// Where pairs are faster than one CTA per 128 x 128 tile, from sweeps of M 136 .. 4096, N 512 .. 28672, K 512 .. 8192: a round of pairs
+// (one 256 x 256 tile each) takes 1.66 - 1.77 times as long as a round of single CTAs, so they win where the other kernel needs at
+// least 1.75 times the rounds. 4096 x 28672 x 8192: 1.09 ms against 1.39; 512 x 8192 x 8192 (one round against two): 53 us against 64;
+// but 768 x 8192 x 4096 (two against three) 48.4 against 41.3 and 640 x 28672 x 4096 (five against eight) 115 against 105. A short
 // reduction is mostly prologue and epilogue: with K 512 and two rounds 136 x 28672 takes 20.3 us against 18.7, from three on pairs are level or ahead.
 bool prefersPair(int M, int N, int K) {
   auto rounds = [](long long tiles, int at) { return (tiles + at - 1) / at; };
   const long long two = rounds((long long)((M + BT - 1) / BT) * ((N + BT - 1) / BT), gemm2::pairsOnDevice());
   const long long one = rounds((long long)((M + 127) / 128) * ((N + 127) / 128), gemm::smCount());
-  return 3 * two <= 2 * one && (K >= 1024 || two >= 3);
+  return 7 * two <= 4 * one && (K >= 1024 || two >= 3);
 }
 
 // C [M, N or N / 2] = A8 [M, K] * B8 [N, K]^T, lda / ldb in bytes; sA[kb * sABlock + row * sARow]. swiglu: B holds 64 gate and 64 up

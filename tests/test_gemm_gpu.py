@@ -81,7 +81,7 @@ def test_gemm_of_few_rows_matches_fp32(M, N, K, wt):
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 128, 128), (1, 1000, 256), (16, 6144, 4096), (17, 136, 384), (32, 4096, 14336), (33, 4096, 1152), (64, 28672, 512),
-                                   (65, 1032, 640), (128, 264, 4096), (192, 512, 8192), (257, 640, 384), (16, 136, 16512)])
+                                   (65, 1032, 640), (65, 1032, 1152), (128, 264, 4096), (192, 512, 8192), (257, 640, 384), (16, 136, 16512), (40, 2056, 640), (20, 6152, 512), (1, 520, 896)])
 def test_fp8_linear_of_few_rows_matches_the_oracle(M, N, K):
     """The block-scaled kernel with output features as MMA rows (one to four token tiles, ragged edges, more splits than blocks of K, a K
     whose scales just do not fit), behind the quantiser it may overlap. Products of codes are exact in fp32; bound: the bf16 rounding of
@@ -146,7 +146,7 @@ def test_quantisers_keep_the_sign_of_zeros_and_of_what_rounds_to_zero(amax):
     comm.destroy()
 
 
-@pytest.mark.parametrize("M,N,K", [(1000, 8200, 1152), (129, 28680, 1152), (513, 8192, 1152), (2049, 8200, 640), (4096, 6144, 512), (4097, 4104, 512)])
+@pytest.mark.parametrize("M,N,K", [(1000, 8200, 1152), (129, 28680, 1152), (513, 8192, 1152), (2049, 8200, 640), (4096, 6144, 512), (4097, 4104, 512), (513, 4232, 1152), (2049, 7176, 640)])
 def test_fp8_gemm_on_cta_pairs_equals_the_one_cta_kernel(M, N, K):
     """Sizes that the rule sends to CTA pairs (ragged rows, columns and an odd number of blocks of K): every partial product is folded in the
     same order with the same operations, so the results are bit-equal to the kernel that a CTA limit asks for. Strided output; nothing else is written."""

@@ -72,5 +72,5 @@ def test_tensor_parallel_mlp_on_one_rank_at_the_plain_gemms_sizes(fused):
     """Sizes that the plain CTA-pair GEMMs with the SwiGLU epilogue take on one rank (more than a round of 256 x 256 tiles, an odd number of
     128-row blocks, a reduction that is no multiple of 256)."""
     _tp(fused, 29890, "tp_worker.py", "--rows", "640", "--hidden", "1152", "--ffn", "4224", fused_kernels="agGemmKernel,gemmRsKernel", plain_kernels="gemmPairKernel")
-    _tp(fused, 29891, "tp_worker.py", "--fp8", "--rows", "1152", "--hidden", "1152", "--ffn", "4224", fused_kernels="agGemmFp8Kernel,gemmRsFp8Kernel",
+    _tp(fused, 29891, "tp_worker.py", "--fp8", "--rows", "1152", "--hidden", "1152", "--ffn", "3200", fused_kernels="agGemmFp8Kernel,gemmRsFp8Kernel",
         plain_kernels="gemmFp8PairKernel")
