@@ -286,6 +286,24 @@ ncclResult_t agPullByCopyEngine(Comm* c, ncclComm_t comm, char* xLocal, char* co
   return ncclSuccess;
 }
 
+// Whether the CTA-pair kernel beats this file's one-CTA kernel on one rank, from a sweep of M 384 .. 8192, weight rows 1024 .. 28672, K 1024
+// .. 8192 (us, one CTA against pairs). In as many rounds of tiles it does (4096 x 8192 x 8192 395 against 332). In more rounds it does not
+// while those are few (640 x 7168 x 4096, one against two: 31 against 47; 1152 x 8192 x 4096, two against three: 61 against 67);
+// from three against four on its better reuse of wide weights makes up for it (1664 x 8192 x 8192 175 against 187, but 384 x
+// 28672 x 4096 111 against 94; 1152 x 16384 x 4096, four against five: 137 against 116). Its SwiGLU epilogue is longer than a short
+// main loop (4096 x 8192 x 1024 97 against 100, 640 x 4096 x 1024 17.2 against 17.8) and wants gate and up rows in turn per 128. Weight
+// rows that are no multiple of 256 make the one-CTA tiles half as large, so pairs must save a round (640 x 640 x 4096 26.6 against 30.4).
+bool pairsOnOneRank(int M, int wRows, int K, bool swiglu) {
+  auto rounds = [](int tiles, int at) { return (tiles + at - 1) / at; };
+  const int bn = wRows % 256 == 0 ? 256 : 128;
+  const int two = rounds((M + 255) / 256 * ((wRows + 255) / 256), gemm2::pairsOnDevice()), one = rounds(M / BM * (wRows / bn), smCount());
+  if (bn == 128) return !swiglu && two < one;
+  if (swiglu && K <= 1024) return false;
+  if (two <= one) return true;
+  const bool shortSwiglu = swiglu && K < 4096;
+  return (one >= 4 && !shortSwiglu) || (one >= 3 && wRows > (shortSwiglu ? 12288 : 8192));
+}
+
 ncclResult_t rsNextCall(Comm* c, const void* workspace, int tileW, unsigned long long* calls) {
   addReleaseNotifier(tpForget);
   std::lock_guard<std::mutex> lk(gTpMu);
@@ -317,18 +335,18 @@ ncclResult_t b200collAgGemm(ncclComm_t comm, void* xSym, const void* w, void* ou
   if (!xSym || !w || !out) BFAIL(ncclInvalidArgument, "b200collAgGemm: null buffer");
   if (rowsPerRank <= 0 || rowsPerRank % BM) BFAIL(ncclInvalidArgument, "b200collAgGemm: rows per rank (%d) must be a multiple of %d", rowsPerRank, BM);
   if (K % 8 || wRows % 128) BFAIL(ncclInvalidArgument, "b200collAgGemm: K %% 8 and weight rows %% 128 must be 0");
+  if ((uintptr_t)out & 15) BFAIL(ncclInvalidArgument, "b200collAgGemm: the output must be 16-byte aligned");
   const int bn = (wRows % 256 == 0) ? 256 : 128;
   const int M = rowsPerRank * n;
   if (c->asyncError.load() != ncclSuccess) BFAIL((ncclResult_t)c->asyncError.load(), "communicator is in an error state: %s", c->lastErr.c_str());
   DevGuard2 g(c->cudaDev);
-  // One rank gathers nothing: the plain GEMMs take the call where they have its epilogue. Without SwiGLU that is the CTA-pair
-  // kernel (4096 x 4096 x 6144: 0.14 ms against 0.16 for the one-CTA kernel below); with it the few-row kernel, whose rule
-  // says where (128 x 28672 x 4096: 47 us against 49.5, and half the device stays idle on smaller weights), else CTA pairs if
-  // gate and up rows take turns per 128.
-  if (plainOnOneRank(n) && (!swiglu || bn == 256 || gemmn::prefersNarrow(M, wRows, K))) {
+  // One rank gathers nothing: the plain GEMMs take the call where they are faster than the one-CTA kernel below.
+  const bool narrow = gemmn::prefersNarrow(M, wRows, K);
+  const bool pairs = pairsOnOneRank(M, wRows, K, swiglu != 0);
+  if (plainOnOneRank(n) && (narrow || pairs)) {
     cudaError_t e;
     if (!swiglu) e = gemm2::gemmPairBf16(xSym, w, out, M, wRows, K, K, K, wRows, false, false, 0, 0, stream);
-    else if (gemmn::prefersNarrow(M, wRows, K)) e = gemmn::gemmNarrowBf16(xSym, w, out, M, wRows, K, K, K, wRows / 2, false, bn, stream);
+    else if (narrow) e = gemmn::gemmNarrowBf16(xSym, w, out, M, wRows, K, K, K, wRows / 2, false, bn, stream);
     else e = gemm2::gemmPairSwiglu(xSym, w, out, M, wRows, K, stream);
     if (e == cudaErrorInvalidValue) BFAIL(ncclInvalidArgument, "b200collAgGemm: operands must be 16-byte aligned with rows a multiple of 16 bytes");
     if (e != cudaSuccess) BFAIL(ncclUnhandledCudaError, "b200collAgGemm launch failed: %s", cudaGetErrorString(e));
