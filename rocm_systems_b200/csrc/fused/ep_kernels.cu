@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(256) epCombine(const __grid_constant__ Combine
 //   epGateGrad    home rank: d gate[t, r] = <dy[t], expert output row of (t, r)>, the row pulled from its owner as in combine.
 //   epGatherGrad  expert's rank: for every row that arrived, pull dy of its token from the token's home rank and scale it
 //                 by the token's gate weight there: the gradient with respect to the expert's output row.
-// The expert GEMMs' gradients are grouped GEMMs on the transposed weights (b200collEpGroupedGemm); the input gradient is
+// The expert GEMMs' gradients are grouped GEMMs that read weights and rows as they lie (b200collEpExpertsBackward); the input gradient is
 // epCombine with unit weights over the rows the last grouped GEMM left in the window's output region.
 struct GateGradArgs {
   const __nv_bfloat16* dy;  // [T, hidden]
@@ -838,8 +838,7 @@ ncclResult_t b200collEpCombine(ncclComm_t comm, void* winSym, const int* topIdx,
 // ---- backward pass ---------------------------------------------------------------------------------------------
 // out[rows of expert e] = a[rows of expert e] * w[e]^T for every local expert, over the rows of the latest dispatch:
 // a [expertsLocal * cap, K], w [expertsLocal * wRows, K], out [expertsLocal * cap, wRows] (nullptr: the window's output
-// region, which needs wRows == hidden). Row blocks without tokens are skipped. The three GEMMs of the experts' backward
-// pass (and the recomputation of the gate/up pre-activations) are calls of this with transposed weights.
+// region, which needs wRows == hidden). Row blocks without tokens are skipped.
 ncclResult_t b200collEpGroupedGemm(ncclComm_t comm, void* winSym, const void* a, const void* w, void* out, int wRows, int K, int expertsLocal, int cap,
                                    int hidden, int ffn, cudaStream_t stream) {
   Comm* c = asComm(comm);

@@ -132,7 +132,6 @@ __device__ __forceinline__ void drainStaged(uint8_t* sw, int lane, int outCols, 
 
 // Policy interface (all __device__):
 //   void coord(int t, int tilesM, int tilesN, int& tm, int& tn)        tile order
-//   bool valid(int tm, int tn)                                         false: the tile is skipped by every role
 //   int aRow(int tm), int bRow(int tm, int tn)                         first row of the tile in the A / B tensor maps
 //   bool waitTile(int tm, int tn, volatile int* err)                   producer: operands of the tile are in place
 //   void drain(uint32_t taddr, int tm, int tn, int q, int lane, uint8_t* sw)  epilogue warp q: read its 32 accumulator rows at taddr (+column)
@@ -189,7 +188,6 @@ __device__ __forceinline__ void gemmCta(const Params& p, Policy& pol, int cta, i
       for (int t = cta; t < numTiles && ok; t += nctas) {
         int tm, tn;
         pol.coord(t, p.tilesM, p.tilesN, tm, tn);
-        if (!pol.valid(tm, tn)) continue;
         if (!pol.waitTile(tm, tn, err)) { ok = false; break; }
         const int aRow = pol.aRow(tm), bRow = pol.bRow(tm, tn);
         for (int k = 0; k < kIters; k++) {
@@ -216,7 +214,6 @@ __device__ __forceinline__ void gemmCta(const Params& p, Policy& pol, int cta, i
         {
           int tm, tn;
           pol.coord(t, p.tilesM, p.tilesN, tm, tn);
-          if (!pol.valid(tm, tn)) continue;
         }
         const int b = it & 1;
         const uint32_t accPhase = (it >> 1) & 1;
@@ -245,7 +242,6 @@ __device__ __forceinline__ void gemmCta(const Params& p, Policy& pol, int cta, i
     for (int t = cta; t < numTiles && ok; t += nctas) {
       int tm, tn;
       pol.coord(t, p.tilesM, p.tilesN, tm, tn);
-      if (!pol.valid(tm, tn)) continue;
       const int b = it & 1;
       const uint32_t accPhase = (it >> 1) & 1;
       it++;
@@ -269,7 +265,6 @@ template <int BN> struct PlainPolicy {
   int ldc;
   int N;
   __device__ __forceinline__ void coord(int t, int tilesM, int tilesN, int& tm, int& tn) const { bandedCoord(t, tilesM, tilesN, tm, tn); }
-  __device__ __forceinline__ bool valid(int, int) const { return true; }
   __device__ __forceinline__ int aRow(int tm) const { return tm * BM; }
   __device__ __forceinline__ int bRow(int, int tn) const { return tn * BN; }
   __device__ __forceinline__ bool waitTile(int, int, volatile int*) const { return true; }

@@ -181,6 +181,7 @@ __device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.
 __device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Arrive on a barrier of any CTA of the cluster. What it orders are tensor-memory accesses, through the tcgen05 fences on both sides,
 // and no memory writes: the default release at CTA scope, as a cluster-scope release waits several hundred cycles for nothing.
+// So nothing else may be handed over through this arrival: data in shared or global memory for another CTA needs a release of cluster scope.
 __device__ __forceinline__ void mbarArriveCluster(uint32_t clusterAddr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(clusterAddr) : "memory");
 }

@@ -52,7 +52,6 @@ template <int BN, bool SWIGLU> struct AgPolicy {
     tm = owner * a.blocksPerRank + r / tilesN;
     tn = r % tilesN;
   }
-  __device__ __forceinline__ bool valid(int, int) const { return true; }
   __device__ __forceinline__ int aRow(int tm) const { return tm * BM; }
   __device__ __forceinline__ int bRow(int, int tn) const { return tn * BN; }
   __device__ __forceinline__ bool waitTile(int tm, int, volatile int* err) const {
@@ -142,7 +141,6 @@ template <int BN> struct RsPolicy {
     tm = owner * a.blocksPerRank + r / tilesN;
     tn = r % tilesN;
   }
-  __device__ __forceinline__ bool valid(int, int) const { return true; }
   __device__ __forceinline__ int aRow(int tm) const { return tm * BM; }
   __device__ __forceinline__ int bRow(int, int tn) const { return tn * BN; }
   __device__ __forceinline__ bool waitTile(int, int, volatile int*) const { return true; }

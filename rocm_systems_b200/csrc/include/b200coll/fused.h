@@ -33,7 +33,8 @@ ncclResult_t b200collAgGemm(ncclComm_t comm, void* xSym, const void* w, void* ou
  * a [nranks * rowsPerRank, K] bf16 and w [N, K] bf16 are this rank's K-shards; y [rowsPerRank, N]
  * bf16 receives rows [rank * rowsPerRank, +rowsPerRank) of sum_over_ranks(a * w^T).
  * workspaceSym: zero-initialised symmetric memory of b200collGemmRsWorkspaceBytes() bytes, the
- * same allocation on every call of a sequence. */
+ * same allocation on every call of a sequence. y overlaps none of the inputs: tiles of it are written while others are computed.
+ * On one rank the plain GEMM kernels write y and the workspace is not used; y and the output of AgGemm are 16-byte aligned. */
 size_t b200collGemmRsWorkspaceBytes(int rowsPerRank, int N, int nranks);
 ncclResult_t b200collGemmRs(ncclComm_t comm, const void* a, const void* w, void* workspaceSym, void* y, int rowsPerRank, int N, int K,
                             cudaStream_t stream);
