@@ -7,6 +7,7 @@ Cases (inputs are larger than the 126 MB L2 where the kernel streams memory, and
 
     gemm        the CTA-pair tcgen05 GEMM in its three operand orders and the one-CTA kernel, 4096 x 4096 x 4096
     fp8         block-scaled e4m3 GEMM and its two quantisers, 4096 x 4096 x 4096
+    decode      the few-row GEMMs in bf16 and e4m3 (with the quantiser in front), 16 and 128 rows against 28672 x 4096 / 8192
     tp          fused all-gather->GEMM(+SwiGLU) and GEMM->reduce-scatter on a communicator of one rank (tiles, policies,
                 epilogues, staging and reducer run as on many ranks; nothing crosses a link). One rank on its own takes the
                 plain GEMMs instead, so this case sets B200COLL_FUSED_ONE_RANK=1 unless the environment says otherwise
@@ -74,6 +75,22 @@ def case_fp8(iters: int) -> dict:
     wq, ws = fp8.quantize_weight(w)
     out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
     res["gemm_fp8_ms"] = _time(lambda: fp8.gemm(xq, xs, wq, ws, out=out), iters)
+    res["gemm_error"] = ops.gemm_take_error()
+    return res
+
+
+def case_decode(iters: int) -> dict:
+    from ..ops import fp8
+    from ..ops import train_ops as ops
+
+    res = {}
+    w = (torch.randn(28672, 4096, device="cuda") * 0.02).to(torch.bfloat16)
+    wq, ws = fp8.quantize_weight((torch.randn(28672, 8192, device="cuda") * 0.02).to(torch.bfloat16))
+    for rows in (16, 128):
+        x = torch.randn(rows, 4096, device="cuda").to(torch.bfloat16)
+        res[f"bf16_{rows}_rows_ms"] = _time(lambda: ops.gemm(x, w), iters)
+    x = torch.randn(16, 8192, device="cuda").to(torch.bfloat16)
+    res["fp8_linear_16_rows_ms"] = _time(lambda: fp8.linear(x, wq, ws), iters)
     res["gemm_error"] = ops.gemm_take_error()
     return res
 
@@ -181,7 +198,7 @@ def case_emu(iters: int) -> dict:
     return res
 
 
-CASES = {"gemm": case_gemm, "fp8": case_fp8, "tp": case_tp, "ep": case_ep, "train": case_train, "emu": case_emu}
+CASES = {"gemm": case_gemm, "fp8": case_fp8, "decode": case_decode, "tp": case_tp, "ep": case_ep, "train": case_train, "emu": case_emu}
 
 
 def main() -> int:

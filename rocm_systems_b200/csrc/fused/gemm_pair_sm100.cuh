@@ -25,9 +25,9 @@
 //   kRows  C[rows of e] = A[rows of e] * B_e^T over the 256-row blocks that hold tokens.
 //   kSum   C_e[M, N] = A[rows of e]^T * B[rows of e] (a weight gradient), reduced over the rows that hold tokens; the rows up to the
 //          next multiple of 16 must be zeros in both operands.
-// 32 experts, 4096 tokens, top-8, hidden 4096, ffn 1024: the two weight gradients 0.69 ms (64 launches of the plain form 1.11 ms), the
-// four kRows GEMMs of a backward pass and its recomputation 1.24 ms (1.32 on one CTA per 128 x 256 tile), the SwiGLU form
-// for 4096 x 28672 x 4096 0.58 ms (1.00).
+// 32 experts, 4096 tokens, top-8, hidden 4096, ffn 1024, forward and backward (seven launches): the SwiGLU form of the gate/up GEMM 0.40 ms, the
+// down GEMM and the recomputed gate/up GEMM 0.64, the two rows' gradients 0.62, the two weight gradients 0.67 (64 launches of
+// the plain form 1.11). The SwiGLU form for 4096 x 28672 x 4096 0.60 ms (1.00 on one CTA per 128 x 256 tile).
 #pragma once
 
 #include "gemm_sm100.cuh"
